@@ -91,19 +91,29 @@ k_project_grouped_exact(const uint8_t *__restrict__ w, uint32_t rows_e, uint32_t
         for (int t = 0; t < tokens; t++) store_act<YT>(y + (size_t)(first + t0 + t) * rows_e + row, acc[t]);
 }
 
-// y[t][c] = decode(W[ids[t]][c]); grid (tokens, ceil(cols / 256)).
+// y[t][c] = decode(W[ids[t]][c]); grid (tokens, ceil(cols / 1024)), four consecutive values per thread (a block of any
+// format holds a multiple of four, so they share their scales).
 template <int FMT, typename YT>
 __global__ void __launch_bounds__(256)
 k_get_rows(const uint8_t *__restrict__ w, uint32_t rows, uint32_t cols, uint32_t row_bytes,
            const uint32_t *__restrict__ ids, YT *__restrict__ y) {
     constexpr int EL = BlockTraits<FMT>::EL;
-    const uint32_t c = blockIdx.y * 256 + threadIdx.x;
+    const uint32_t c = (blockIdx.y * 256 + threadIdx.x) * 4;
     const uint32_t t = blockIdx.x;
     if (c >= cols) return;
     const uint32_t r = ids[t];
-    // An id beyond the matrix decodes nothing; the row is written as zeros.
-    const float v = r < rows ? decode_at<FMT>(w + (size_t)r * row_bytes, cols / EL, c / EL, c % EL) : 0.f;
-    store_act<YT>(y + (size_t)t * cols + c, v);
+    float v[4] = {0.f, 0.f, 0.f, 0.f}; // an id beyond the matrix decodes nothing; the row is written as zeros
+    if (r < rows) {
+        const uint8_t *row = w + (size_t)r * row_bytes;
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = decode_at<FMT>(row, cols / EL, c / EL, c % EL + i);
+    }
+    YT *dst = y + (size_t)t * cols + c;
+    if constexpr (sizeof(YT) == 4) *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else {
+        const __nv_bfloat162 a = __halves2bfloat162(to_bf16_rne(v[0]), to_bf16_rne(v[1])), b = __halves2bfloat162(to_bf16_rne(v[2]), to_bf16_rne(v[3]));
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+    }
 }
 
 template <typename F> int dispatch_format(fq_device *dev, uint32_t format, F &&f) {
@@ -167,7 +177,7 @@ int fq_launch_project_grouped_exact(fq_device *dev, const ProjectArgs &a) {
 int fq_launch_get_rows(fq_device *dev, const fq_matrix *w, const uint32_t *ids, uint32_t tokens, void *y,
                        int y_dtype) {
     return dispatch_format(dev, w->format, [&](auto fmt) {
-        dim3 grid(tokens, ((uint32_t)w->cols + 255) / 256);
+        dim3 grid(tokens, ((uint32_t)w->cols + 1023) / 1024);
         if (y_dtype == FQ_BF16)
             k_get_rows<decltype(fmt)::value, __nv_bfloat16><<<grid, 256, 0, dev->stream>>>(
                 w->data, (uint32_t)w->rows, (uint32_t)w->cols, (uint32_t)w->pitch, ids, (__nv_bfloat16 *)y);

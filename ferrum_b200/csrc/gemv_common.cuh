@@ -133,21 +133,54 @@ __device__ __forceinline__ Quant8 quantize8(const float (&v)[8]) {
     }
     return q;
 }
-// 1 / sqrt(mean(x^2) + eps) of a row of n values (a multiple of 4), by one warp: every lane sums the float4s
-// lane, lane + 32, .. in order and the lanes are added by a butterfly, so any warp that calls this on the same row
-// gets the same bits (the standalone normalisation and the one fused into activation preparation agree).
-__device__ __forceinline__ float row_inv_rms(const float *__restrict__ row, uint32_t n, float eps, uint32_t lane) {
-    float ss = 0.f;
-    for (uint32_t i = lane; i < n / 4; i += 32) {
-        const float4 v = reinterpret_cast<const float4 *>(row)[i];
-        ss = fmaf(v.x, v.x, ss);
-        ss = fmaf(v.y, v.y, ss);
-        ss = fmaf(v.z, v.z, ss);
-        ss = fmaf(v.w, v.w, ss);
-    }
+// 1 / sqrt(mean(x^2) + eps) of a row of n values (a multiple of 4).  The sum is that of sixteen virtual warps: lane l
+// of virtual warp w adds the float4s 32 w + l, + 512, .. in order, a butterfly adds its lanes, and the sixteen are added
+// in order.  Whoever computes it -- a block of 16 warps, one of four, a single warp -- gets the same bits, so the
+// standalone normalisation and the ones fused into activation preparation agree.  (One warp walking the row in a single
+// chain, as this once was, took 15 us on a 5120-value row: 40 dependent loads.)
+constexpr uint32_t NORM_WARPS = 16;
+__device__ __forceinline__ float norm_square(float ss, const float4 &v) {
+    ss = fmaf(v.x, v.x, ss);
+    ss = fmaf(v.y, v.y, ss);
+    ss = fmaf(v.z, v.z, ss);
+    return fmaf(v.w, v.w, ss);
+}
+__device__ __forceinline__ float norm_butterfly(float ss) {
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+    return ss;
+}
+__device__ __forceinline__ float norm_finish(const float *part, uint32_t n, float eps) {
+    float ss = 0.f;
+#pragma unroll
+    for (uint32_t w = 0; w < NORM_WARPS; w++) ss += part[w];
     return 1.0f / sqrtf(ss / (float)n + eps);
+}
+// By a block of at most sixteen warps (a power of two); `part` holds NORM_WARPS floats of shared memory.  Synchronises.
+__device__ __forceinline__ float block_inv_rms(const float *__restrict__ row, uint32_t n, float eps, float *part) {
+    const uint32_t lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    for (uint32_t w = threadIdx.x >> 5; w < NORM_WARPS; w += warps) {
+        float ss = 0.f;
+#pragma unroll 4
+        for (uint32_t i = 32 * w + lane; i < n / 4; i += 32 * NORM_WARPS) ss = norm_square(ss, reinterpret_cast<const float4 *>(row)[i]);
+        ss = norm_butterfly(ss);
+        if (lane == 0) part[w] = ss;
+    }
+    __syncthreads();
+    return norm_finish(part, n, eps);
+}
+// By one warp.
+__device__ __forceinline__ float row_inv_rms(const float *__restrict__ row, uint32_t n, float eps, uint32_t lane) {
+    float part[NORM_WARPS];
+#pragma unroll
+    for (uint32_t w = 0; w < NORM_WARPS; w++) part[w] = 0.f;
+    for (uint32_t i0 = lane; i0 < n / 4; i0 += 32 * NORM_WARPS)
+#pragma unroll
+        for (uint32_t w = 0; w < NORM_WARPS; w++)
+            if (i0 + 32 * w < n / 4) part[w] = norm_square(part[w], reinterpret_cast<const float4 *>(row)[i0 + 32 * w]);
+#pragma unroll
+    for (uint32_t w = 0; w < NORM_WARPS; w++) part[w] = norm_butterfly(part[w]);
+    return norm_finish(part, n, eps);
 }
 __device__ __forceinline__ uint32_t pack4(const uint8_t *p) { return p[0] | (p[1] << 8) | (p[2] << 16) | ((uint32_t)p[3] << 24); }
 

@@ -123,28 +123,29 @@ __host__ __device__ inline uint32_t nt_act_bytes(uint32_t tok, uint32_t nb) {
     return (tok * (nb * 512 + 64) + tok * nt_rec_stride(nb) + 15u) & ~15u;
 }
 
-// One warp per (activation row, superblock); lane l owns the eight values at 256 b + 8 l.
+// Block (row, run of four superblocks), one warp per superblock; lane l owns the eight values at 256 b + 8 l.
 //   src    (may be null) row i of the prepared set is row src[i] / src_div of x (expert-sorted routes);
 //   range  (may be null) only rows [range[0], range[range_stride]) are prepared (the experts one rank owns);
 //   x_up   (may be null) the activations are the gated unit silu(x) * x_up, as `k_swiglu` computes it;
 //   norm_w (may be null) the activations are rmsnorm(x) * norm_w.
+constexpr uint32_t PREP_WARPS = 4;
 template <int FMT>
-__global__ void __launch_bounds__(128)
-k_prep_nt(const float *__restrict__ x, const float *__restrict__ x_up, const float *__restrict__ norm_w, float eps, uint32_t xrows,
+__global__ void __launch_bounds__(PREP_WARPS * 32)
+k_prep_nt(const float *__restrict__ x, const float *__restrict__ x_up, const float *__restrict__ norm_w, float eps,
           const uint32_t *__restrict__ src, uint32_t src_div, const uint32_t *__restrict__ range, uint32_t range_stride, PrepNT L,
           uint8_t *__restrict__ out) {
     pdl_trigger();
     pdl_wait();
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const uint32_t xr = warp / L.nblk, b = warp % L.nblk;
-    if (xr >= xrows) return;
+    const uint32_t lane = threadIdx.x & 31, xr = blockIdx.x, b = blockIdx.y * PREP_WARPS + (threadIdx.x >> 5);
     if (range && (xr < range[0] || xr >= range[range_stride])) return;
     const size_t srow = src ? src[xr] / src_div : xr;
+    __shared__ float norm_part[NORM_WARPS];
+    const float scale = norm_w ? block_inv_rms(x + srow * L.cols, L.cols, eps, norm_part) : 0.f;
+    if (b >= L.nblk) return;
     const float4 *sp = reinterpret_cast<const float4 *>(x + srow * L.cols + (size_t)b * 256 + lane * 8);
     const float4 v0 = sp[0], v1 = sp[1];
     float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     if (norm_w) { // rmsnorm(x) * norm_w, as `h_rmsnorm` computes it
-        const float scale = row_inv_rms(x + srow * L.cols, L.cols, eps, lane);
         const float4 *ws = reinterpret_cast<const float4 *>(norm_w + (size_t)b * 256 + lane * 8);
         const float4 w0 = ws[0], w1 = ws[1];
         const float g[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
@@ -628,11 +629,11 @@ uint8_t *launch_prep(fq_device *dev, int format, const ProjectArgs &f, uint32_t 
     if ((size_t)xrows * L.token_bytes > dev->xprep_bytes / 2) return nullptr;
     dev->xprep_turn ^= 1u;
     uint8_t *prep = (uint8_t *)dev->xprep + (dev->xprep_turn ? dev->xprep_bytes / 2 : 0);
-    const uint32_t warps = xrows * L.nblk;
+    const dim3 grid(xrows, (L.nblk + PREP_WARPS - 1) / PREP_WARPS);
     if (format == FQ_Q4_K || format == FQ_Q5_K) // the same fragment order
-        e = launch_pdl(k_prep_nt<FQ_Q4_K>, dim3((warps + 3) / 4), dim3(128), 0, dev->stream, (const float *)f.x, f.x_up, f.norm_w, f.norm_eps, xrows, src, src_div, range, range_stride, L, prep);
+        e = launch_pdl(k_prep_nt<FQ_Q4_K>, grid, dim3(PREP_WARPS * 32), 0, dev->stream, (const float *)f.x, f.x_up, f.norm_w, f.norm_eps, src, src_div, range, range_stride, L, prep);
     else
-        e = launch_pdl(k_prep_nt<FQ_Q6_K>, dim3((warps + 3) / 4), dim3(128), 0, dev->stream, (const float *)f.x, f.x_up, f.norm_w, f.norm_eps, xrows, src, src_div, range, range_stride, L, prep);
+        e = launch_pdl(k_prep_nt<FQ_Q6_K>, grid, dim3(PREP_WARPS * 32), 0, dev->stream, (const float *)f.x, f.x_up, f.norm_w, f.norm_eps, src, src_div, range, range_stride, L, prep);
     return prep;
 }
 

@@ -485,12 +485,18 @@ template <typename... Args> void launch_combine(cudaStream_t stream, const float
     else fqk::launch_pdl(k_moe_combine<1>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, args...);
 }
 
-// out = g / (1 + exp(-g)) * u
-__global__ void k_swiglu(const float *__restrict__ g, const float *__restrict__ u, size_t n, float *__restrict__ y) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        const float x = g[i];
-        y[i] = x / (1.f + expf(-x)) * u[i];
+// out = g / (1 + exp(-g)) * u, four values per thread (the remainder one by one)
+__device__ __forceinline__ float swiglu(float x, float u) { return x / (1.f + expf(-x)) * u; }
+__global__ void __launch_bounds__(256)
+k_swiglu(const float *__restrict__ g, const float *__restrict__ u, size_t n, float *__restrict__ y) {
+    fqk::pdl_trigger();
+    fqk::pdl_wait();
+    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (i + 4 <= n) {
+        const float4 a = *reinterpret_cast<const float4 *>(g + i), b = *reinterpret_cast<const float4 *>(u + i);
+        *reinterpret_cast<float4 *>(y + i) = make_float4(swiglu(a.x, b.x), swiglu(a.y, b.y), swiglu(a.z, b.z), swiglu(a.w, b.w));
+    } else {
+        for (size_t j = i; j < n; j++) y[j] = swiglu(g[j], u[j]);
     }
 }
 
@@ -684,6 +690,6 @@ extern "C" int fq_glu(fq_device *dev, const float *gate, const float *up, size_t
     if (int rc = fq_check_binding(dev, gate, n * 4, "gate")) return rc;
     if (int rc = fq_check_binding(dev, up, n * 4, "up")) return rc;
     if (int rc = fq_check_binding(dev, out, n * 4, "out")) return rc;
-    k_swiglu<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>(gate, up, n, out);
+    if (int rc = fq_check_cuda(dev, fqk::launch_pdl(k_swiglu, dim3((unsigned)((n + 1023) / 1024)), dim3(256), 0, dev->stream, gate, up, n, out), "glu launch")) return rc;
     return fq_end_enqueue(dev, "glu", 1);
 }
