@@ -705,6 +705,8 @@ static int check_dtype(fq_device *dev, int dt) {
     return (dt == FQ_F32 || dt == FQ_BF16) ? FQ_OK : fq_fail(dev, FQ_ERR_UNSUPPORTED, "element type %d", dt);
 }
 
+static bool is_iq4(uint32_t format) { return format == FQ_IQ4_NL || format == FQ_IQ4_XS; }
+
 // Decode / verify widths (F32 in and out): Q8_0 on the integer-dot kernel, Q4_K / Q6_K on the integer tensor
 // path -- one activation row (and per-route expert projections) in gemv_i8.cu, 2..16 rows in gemv_nt.cu.
 static int launch_decode(fq_device *dev, const ProjectArgs *a, uint32_t count) {
@@ -712,11 +714,9 @@ static int launch_decode(fq_device *dev, const ProjectArgs *a, uint32_t count) {
         int rc = fq_launch_gemv_q8(dev, a[0]);
         if (rc != FQ_ERR_UNSUPPORTED) return rc;
     }
-    if (count == 1 && (a[0].m == 1 || a[0].ids) && (a[0].format == FQ_IQ4_NL || a[0].format == FQ_IQ4_XS)) { // dense with more rows: the exact kernel measured faster
-        int rc = fq_launch_gemv_iq4(dev, a[0]);
-        if (rc != FQ_ERR_UNSUPPORTED) return rc;
-    }
-    if (a[0].m == 1 || a[0].ids) return fq_launch_gemv_i8_many(dev, a, count);
+    const bool iq4 = is_iq4(a[0].format);
+    if (count == 1 && a[0].ids && iq4) return fq_launch_gemv_iq4(dev, a[0]);
+    if ((a[0].m == 1 && !iq4) || a[0].ids) return fq_launch_gemv_i8_many(dev, a, count);
     return fq_launch_gemv_nt_many(dev, a, count);
 }
 
@@ -1040,7 +1040,7 @@ static int project_gated(fq_device *dev, const fq_matrix *w, const float *g, con
             }
             a.combine = nullptr;
         }
-        const int rc = (ids || rows_x == 1) ? fq_launch_gemv_i8_many(dev, &a, 1) : fq_launch_gemv_nt_many(dev, &a, 1);
+        const int rc = (ids || (rows_x == 1 && !is_iq4(a.format))) ? fq_launch_gemv_i8_many(dev, &a, 1) : fq_launch_gemv_nt_many(dev, &a, 1);
         if (rc != FQ_ERR_UNSUPPORTED) return rc;
     }
     if (int rc = fq_glu(dev, g, u, rows_x * width, act)) return rc;

@@ -18,6 +18,16 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
+// Eight codebook values of the IQ4 formats (iq4_value in blocks.cuh) for the eight 4-bit indices of `n`: nibble i of the
+// low half -> byte i of .x, of the high half -> byte i of .y.  Three bits of an index select from each half of the
+// codebook with a byte permute; the fourth then picks the half, again by a permute.
+__device__ __forceinline__ uint2 iq4_lookup8(uint32_t n) {
+    constexpr uint32_t T0 = 0xBFAD9881u, T1 = 0xF6EADDCFu, T2 = 0x26190D01u, T3 = 0x71594535u; // entries 0-3, 4-7, 8-11, 12-15
+    const uint32_t low3 = n & 0x77777777u, half = ((n >> 1) & 0x44444444u) | 0x32103210u; // selector 4 + i takes byte i of the upper half's value
+    auto pick = [&](uint32_t sel, uint32_t h) { return __byte_perm(__byte_perm(T0, T1, sel), __byte_perm(T2, T3, sel), h); };
+    return make_uint2(pick(low3, half), pick(low3 >> 16, half >> 16)); // a permute reads the low 16 bits of its selector
+}
+
 // u8 (weights) x s8 (activations), 16 rows x 8 columns x 32 k.
 __device__ __forceinline__ void mma_u8s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
@@ -86,6 +96,46 @@ __device__ __forceinline__ int byte_s(uint32_t w, int i) {
     return r;
 }
 __device__ __forceinline__ uint32_t word_of(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// Eight activations of one lane as 24-bit integers x' = round(x * s) = 65536 hi + 256 mid + lo, all three signed bytes, s
+// the largest power of two with max|x| * s <= 8355711 over the superblock: what fp32 holds of the largest value and at
+// least 2^-24 of it for the others.  Non-finite superblocks as in Quant8 below.
+struct Quant8Wide {
+    uint8_t hi[8], mid[8], lo[8];
+    int e;
+    bool finite;
+};
+__device__ __forceinline__ Quant8Wide quantize8_wide(const float (&v)[8]) {
+    Quant8Wide q;
+    float amax = 0.f;
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        amax = fmaxf(amax, fabsf(v[i]));
+        bad |= !(fabsf(v[i]) < INFINITY);
+    }
+    q.finite = __ballot_sync(0xffffffffu, bad) == 0u;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    int e = 0;
+    if (amax > 0.f && q.finite) {
+        int ex;
+        frexpf(amax, &ex);
+        e = max(-110, min(110, 23 - ex));
+        if (ldexpf(amax, e) > 8355711.f) e -= 1;
+    }
+    q.e = e;
+    const float s = ldexpf(1.f, e);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int x = q.finite ? __float2int_rn(fminf(fmaxf(v[i] * s, -8355711.f), 8355711.f)) : 0;
+        const int m = (x + 128) >> 8, h = (m + 128) >> 8;
+        q.lo[i] = (uint8_t)(x - (m << 8));
+        q.mid[i] = (uint8_t)(m - (h << 8));
+        q.hi[i] = (uint8_t)h;
+    }
+    return q;
+}
 
 // Eight activations of one lane (values 8 lane .. 8 lane + 7 of a 256-value superblock handled by one warp) as
 // 16-bit integers x' = round(x * s) = 256 hi + lo with both halves signed bytes; s = 2^e is the largest power of
@@ -242,12 +292,17 @@ __device__ __forceinline__ void tp_finish(const TpPush &P, uint32_t seq) {
 // block-wide barrier.  A stage holds one superblock of 16 rows, row r at r * ROW (ROW >= the bytes of a row's
 // superblock, padded so that the reads of a kernel's fragment pattern fall on different banks):
 //   Q4_K / Q5_K  the 144 / 176 bytes of the block;
+//   IQ4          the 128 bytes of nibbles, then the superblock's scales: IQ4_XS 8 bytes d | scales_h | scales_l, IQ4_NL
+//                the eight f16 d of its blocks;
 //   Q6_K         ql[128] | qh[64] | scales[16] of the device layout (blocks.cuh), and after the 16 rows 4 bytes
 //                per row: the aligned word that holds the f16 d of the superblock (its high half for odd b).
 // A lane copies the same pieces of every superblock, so their offsets from the tile's first row are worked out
 // once per tile (`start_tile`); rows past the end of the matrix read its last row.
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void *smem_dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async4(void *smem_dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(src) : "memory");
@@ -256,18 +311,21 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <int FMT, uint32_t ROW> struct WeightRing {
-    static constexpr uint32_t SRC = FMT == FQ_Q4_K ? 144 : FMT == FQ_Q5_K ? 176 : 208; // bytes copied per row and superblock
+    static constexpr bool IQ4 = FMT == FQ_IQ4_XS || FMT == FQ_IQ4_NL;
+    static constexpr uint32_t SRC = FMT == FQ_Q4_K ? 144 : FMT == FQ_Q5_K ? 176 : IQ4 ? 144 : 208; // bytes copied per row and superblock
     static constexpr uint32_t PER_ROW = SRC / 16;
     static constexpr uint32_t PIECES = 16 * PER_ROW;
-    static constexpr int NP = FMT == FQ_Q6_K ? 7 : (int)((PIECES + 31) / 32);
+    static constexpr int NP = FMT == FQ_Q6_K ? 7 : IQ4 ? 5 : (int)((PIECES + 31) / 32);
     static constexpr uint32_t BYTES = 16 * ROW + (FMT == FQ_Q6_K ? 64 : 0);
     static_assert(ROW >= SRC && ROW % 16 == 0, "stage rows hold a row's superblock and stay 16-byte aligned");
     const uint8_t *base = nullptr;
     uint32_t off[NP];
     // Q6_K: pieces 0..127 are ql (row p / 8), 128..191 qh (row / 4), 192..207 the scales, 208..223 the word with d.
+    // IQ4: pieces 0..127 are nibbles (row p / 8), then one piece of scales per row (lanes 0..15).
     __device__ __forceinline__ uint32_t piece_row(int i, uint32_t lane) const {
         const uint32_t p = lane + 32 * i;
-        if constexpr (FMT != FQ_Q6_K) return p / PER_ROW;
+        if constexpr (IQ4) return i < 4 ? p / 8 : (lane & 15);
+        else if constexpr (FMT != FQ_Q6_K) return p / PER_ROW;
         return i < 4 ? p / 8 : i < 6 ? (p - 128) / 4 : (lane & 15);
     }
     // `first_row`: the tile's first weight row; `last`: index of the matrix's last row relative to it.
@@ -277,7 +335,8 @@ template <int FMT, uint32_t ROW> struct WeightRing {
         for (int i = 0; i < NP; i++) {
             const uint32_t p = lane + 32 * i, r = min(piece_row(i, lane), last);
             uint32_t in_row;
-            if constexpr (FMT != FQ_Q6_K) in_row = 16 * (p % PER_ROW);
+            if constexpr (IQ4) in_row = i < 4 ? 16 * (p % 8) : nblk * 128;
+            else if constexpr (FMT != FQ_Q6_K) in_row = 16 * (p % PER_ROW);
             else in_row = i < 4 ? 16 * (p % 8) : i < 6 ? nblk * 128 + 16 * (p % 4) : lane < 16 ? nblk * 192 : nblk * 208;
             off[i] = r * pitch + in_row;
         }
@@ -287,7 +346,13 @@ template <int FMT, uint32_t ROW> struct WeightRing {
 #pragma unroll
         for (int i = 0; i < NP; i++) {
             const uint32_t p = lane + 32 * i;
-            if constexpr (FMT != FQ_Q6_K) {
+            if constexpr (IQ4) {
+                if (i < 4) cp_async16(dst + ROW * (p / 8) + 16 * (p % 8), base + (off[i] + b * 128));
+                else if (lane < 16) {
+                    if constexpr (FMT == FQ_IQ4_XS) cp_async8(dst + ROW * lane + 128, base + (off[i] + b * 8));
+                    else cp_async16(dst + ROW * lane + 128, base + (off[i] + b * 16));
+                }
+            } else if constexpr (FMT != FQ_Q6_K) {
                 if (p < PIECES) cp_async16(dst + ROW * (p / PER_ROW) + 16 * (p % PER_ROW), base + (off[i] + b * SRC));
             } else {
                 if (i < 4) cp_async16(dst + ROW * (p / 8) + 16 * (p % 8), base + (off[i] + b * 128));
