@@ -298,8 +298,8 @@ extern "C" int fq_device_create(int ordinal, fq_device **out) {
     if ((e = cudaMalloc((void **)&dev->side_nt_counters, (size_t)dev->side_nt_counter_count * 4)) != cudaSuccess) return bail(e, "slice counters");
     if ((e = cudaMemset(dev->nt_counters, 0, (size_t)dev->nt_counter_count * 4)) != cudaSuccess) return bail(e, "slice counters");
     if ((e = cudaMemset(dev->side_nt_counters, 0, (size_t)dev->side_nt_counter_count * 4)) != cudaSuccess) return bail(e, "slice counters");
-    if ((e = cudaMalloc((void **)&dev->combine_counters, (size_t)FQ_COMBINE_COUNTERS * 4)) != cudaSuccess) return bail(e, "combine counters");
-    if ((e = cudaMemset(dev->combine_counters, 0, (size_t)FQ_COMBINE_COUNTERS * 4)) != cudaSuccess) return bail(e, "combine counters");
+    if ((e = cudaMalloc((void **)&dev->combine_counters, (size_t)(FQ_COMBINE_COUNTERS + FQ_BARRIER_WORDS) * 4)) != cudaSuccess) return bail(e, "combine counters");
+    if ((e = cudaMemset(dev->combine_counters, 0, (size_t)(FQ_COMBINE_COUNTERS + FQ_BARRIER_WORDS) * 4)) != cudaSuccess) return bail(e, "combine counters");
     if ((e = cudaMalloc(&dev->staging_dev, FQ_HOST_STAGING_BYTES)) != cudaSuccess) return bail(e, "device staging");
     if ((e = cudaMallocHost(&dev->staging_host, FQ_HOST_STAGING_BYTES)) != cudaSuccess) return bail(e, "pinned staging");
     dev->gemm_ws_bytes = (size_t)96 << 20;
@@ -390,7 +390,7 @@ extern "C" int fq_device_recover(fq_device *dev) {
     cudaError_t e = cudaStreamSynchronize(dev->stream);
     if (e != cudaSuccess) return fq_fail(dev, FQ_ERR_SYNC, "stream is still failing: %s", cudaGetErrorString(e));
     // A kernel that gave up a wait may have left arrival counters behind.
-    if (cudaMemset(dev->combine_counters, 0, (size_t)FQ_COMBINE_COUNTERS * 4) != cudaSuccess) cudaGetLastError();
+    if (cudaMemset(dev->combine_counters, 0, (size_t)(FQ_COMBINE_COUNTERS + FQ_BARRIER_WORDS) * 4) != cudaSuccess) cudaGetLastError();
     dev->failed = false;
     dev->error.clear();
     return FQ_OK;
@@ -1166,6 +1166,19 @@ extern "C" int fq_moe_ffn(fq_device *dev, const fq_moe_ffn_desc *f, const float 
     MoeScratch s = moe_layout(f, m, scratch);
     if (scratch_elems < s.total) return fq_fail(dev, FQ_ERR_SHAPE, "MoE scratch holds %zu of %zu floats", scratch_elems, s.total);
     const size_t routes = m * used;
+    if (m == 1 && !dev->exact) {
+        // One token: the whole block is one launch where the shapes have it.
+        if (int rc = fq_begin_enqueue(dev)) return rc;
+        if (int rc = fq_check_binding(dev, x, hidden * 4, "x")) return rc;
+        if (int rc = fq_check_binding(dev, scratch, s.total * 4, "scratch")) return rc;
+        if (int rc = fq_check_binding(dev, out, hidden * 4, "out")) return rc;
+        if (f->shared_gate_inp)
+            if (int rc = fq_check_binding(dev, f->shared_gate_inp, hidden * 4, "shared gate weight")) return rc;
+        if (int rc = fq_check_no_alias(dev, scratch, s.total * 4, x, hidden * 4, "scratch")) return rc;
+        const int rc = fq_launch_moe_decode(dev, f, x, s.logits, s.g, s.u, s.shared_tmp, s.shared_tmp + f->shared_ffn, out);
+        if (rc == FQ_OK) fq_note_write(dev, out, hidden * 4);
+        if (rc != FQ_ERR_UNSUPPORTED) return rc;
+    }
     const bool identity = routes <= MV_ID_MAX_ROUTES || dev->exact;
     // The shared expert depends on x only and runs on the side stream beside the routed chain: at decode widths
     // (small kernels, latency-bound) from the start; at wide inputs after the router, whose GEMM shares the

@@ -22,6 +22,7 @@
 #include <cstdlib>
 
 #include "blocks.cuh"
+#include "gemv_q8.cuh"
 #include "internal.h"
 
 namespace {
@@ -53,25 +54,8 @@ k_gemv_q8(const uint8_t *__restrict__ w, uint32_t rows, uint32_t cols, uint32_t 
     // 1. Activations -> 16-bit integers, one warp per (activation row, block of 32), lane = value.
     for (uint32_t i = warp; i < MT * nb; i += WARPS) {
         const uint32_t mrow = i / nb, b = i % nb;
-        const float v = x[(size_t)mrow * cols + 32 * b + lane];
-        float amax = fabsf(v);
-        const bool finite = __ballot_sync(0xffffffffu, !(fabsf(v) < INFINITY)) == 0u;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-        // s = 2^e, the largest power of two with amax * s <= 32639: amax = f * 2^ex with f in [0.5, 1), so
-        // e = 15 - ex, one less when f * 2^15 > 32639.  Exponents straight from the float's bits.
-        int e = 0;
-        if (amax > 0.f && finite) {
-            const int ex = (int)(__float_as_uint(amax) >> 23) - 126;
-            e = max(-110, min(110, 15 - ex));
-            if (amax * __uint_as_float((uint32_t)(127 + e) << 23) > 32639.f) e -= 1;
-        }
-        int q = __float2int_rn(fminf(fmaxf(v * __uint_as_float((uint32_t)(127 + e) << 23), -32639.f), 32639.f));
-        if (!finite) q = 0; // the block's factor below is NaN in that case
-        const int h = (q + 128) >> 8;
-        hi[(size_t)mrow * cols + 32 * b + lane] = (int8_t)h;
-        lo[(size_t)mrow * cols + 32 * b + lane] = (int8_t)(q - (h << 8));
-        if (lane == 0) isc[mrow * nb + b] = finite ? __uint_as_float((uint32_t)(127 - e) << 23) : __int_as_float(0x7fc00000);
+        fqk::q8_quantize_block(x[(size_t)mrow * cols + 32 * b + lane], lane, hi + (size_t)mrow * cols + 32 * b, lo + (size_t)mrow * cols + 32 * b,
+                               isc + mrow * nb + b);
     }
     __syncthreads();
 
@@ -107,11 +91,7 @@ k_gemv_q8(const uint8_t *__restrict__ w, uint32_t rows, uint32_t cols, uint32_t 
                 const float s = live ? isc[t * nb + b] : 0.f; // lanes past the row's end contribute nothing
 #pragma unroll
                 for (int r = 0; r < RPW; r++) {
-                    int dh = __dp4a((int)q[r].x, xh.x, 0), dl = __dp4a((int)q[r].x, xl.x, 0);
-                    dh = __dp4a((int)q[r].y, xh.y, dh), dl = __dp4a((int)q[r].y, xl.y, dl);
-                    dh = __dp4a((int)q[r].z, xh.z, dh), dl = __dp4a((int)q[r].z, xl.z, dl);
-                    dh = __dp4a((int)q[r].w, xh.w, dh), dl = __dp4a((int)q[r].w, xl.w, dl);
-                    acc[r][t] = fmaf((float)(dh * 256 + dl), d[r] * s, acc[r][t]);
+                    acc[r][t] = fmaf((float)fqk::q8_dot16(q[r], xh, xl), d[r] * s, acc[r][t]);
                 }
             }
         }

@@ -68,7 +68,7 @@ struct fq_device {
     void *nt_ws = nullptr, *side_nt_ws = nullptr;
     size_t nt_ws_bytes = 0, side_nt_ws_bytes = 0;
     uint32_t *nt_counters = nullptr, *side_nt_counters = nullptr;
-    uint32_t *combine_counters = nullptr; // FQ_COMBINE_COUNTERS words, zero between launches
+    uint32_t *combine_counters = nullptr; // FQ_COMBINE_COUNTERS + FQ_BARRIER_WORDS words, zero between launches
     uint32_t nt_counter_count = 0, side_nt_counter_count = 0;
     // Split-K workspace of the prefill GEMM: partial fp32 tiles and one arrival counter per tile.
     float *gemm_ws = nullptr;
@@ -115,6 +115,7 @@ inline size_t fq_dtype_size(int dtype) { return dtype == FQ_BF16 ? 2 : 4; }
 // `h_moe_combine` (src/metal/shaders/hybrid.metal:2371-2388) carried out by the down projection of per-route
 // experts: the last of a token's `used` route blocks to finish a 16-row tile adds the routes' rows in route order.
 constexpr uint32_t FQ_COMBINE_COUNTERS = 8192;
+constexpr uint32_t FQ_BARRIER_WORDS = 4; // after them: the barrier counters of the one-launch MoE block
 struct CombineTail {
     const float *weights, *shared, *gate; // [tokens][used], [tokens][hidden], [tokens]
     float *out;                           // [tokens][hidden]
@@ -159,6 +160,10 @@ constexpr size_t FQ_GEMV_SCRATCH_BYTES = (size_t)96 << 20;
 // Integer tensor-core decode GEMV for one activation row and for per-route expert projections; several
 // matrices of one format and width sharing x in one launch.
 int fq_launch_gemv_i8_many(fq_device *dev, const ProjectArgs *a, uint32_t count);
+// How that kernel cuts K (what a kernel that must return the same bits follows): the contiguous slices of a one-row
+// projection of `tiles` 16-row tiles, and the ways a per-route projection deals the superblocks out.
+uint32_t fq_gemv_i8_slices(const fq_device *dev, uint32_t tiles, uint32_t nblk);
+uint32_t fq_gemv_i8_split(const fq_device *dev, uint32_t tiles, uint32_t routes, uint32_t nblk);
 // The same for 2..16 activation rows (activation rows on the MMA's N side).
 int fq_launch_gemv_nt_many(fq_device *dev, const ProjectArgs *a, uint32_t count);
 // Grouped expert projection over expert-sorted rows (a[i].offsets / slots / groups) for one or two expert stacks
@@ -183,6 +188,9 @@ int fq_launch_moe_gather_bf16(fq_device *dev, const float *x, const uint32_t *so
 int fq_moe_route_map(fq_device *dev, const float *logits, const float *x, const float *shared_w, uint32_t experts, uint32_t used,
                      uint32_t hidden, uint32_t tokens, int sigmoid, int norm, int shared_gate, uint32_t *ids, float *weights, float *gate,
                      uint32_t *offsets, uint32_t *sorted, uint32_t *position);
+// The MoE block of one token in one launch (moe_decode.cu); FQ_ERR_UNSUPPORTED when the shapes or formats have none.
+int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *x, float *logits, float *g, float *u, float *shared_g, float *shared_u,
+                         float *out);
 int fq_launch_glu_bf16(fq_device *dev, const float *gate, const float *up, size_t n, const uint32_t *range, uint32_t stride, uint32_t width,
                        void *out);
 // out[row] = expert of expert-sorted row `row` minus `first`, or an id that names no expert when it is not one

@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 
 #include "gemv_common.cuh"
+#include "moe_route.cuh"
 #include "internal.h"
 
 namespace {
@@ -29,8 +30,23 @@ __device__ __forceinline__ void route_token(float *route_smem, const float *__re
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t t = blockIdx.x * ROUTE_WARPS + warp;
     if (t >= tokens) return;
-    float *prob = route_smem + (size_t)warp * experts;
     const float *row = logits + (size_t)t * experts;
+    if (used <= 32) { // what every model has; the scores stay in registers
+        uint32_t id = 0;
+        float weight = 0.f;
+        const bool good = experts <= 256 ? fqk::route_row<8>(row, experts, used, sigmoid, norm, lane, id, weight)
+                                         : fqk::route_row<32>(row, experts, used, sigmoid, norm, lane, id, weight);
+        // A NaN or an infinity among the logits has no ranking: as below.
+        if (!good && lane == 0) *(volatile int *)status = (int)FQ_ERR_WEIGHT;
+        if (lane < used) {
+            ids[(size_t)t * used + lane] = good ? id : lane;
+            weights[(size_t)t * used + lane] = good ? weight : 0.f;
+        }
+        const float gv = shared_gate && good ? fqk::route_gate(x + (size_t)t * hidden, shared_w, hidden, lane) : good ? 1.f : 0.f;
+        if (lane == 0) gate[t] = gv;
+        return;
+    }
+    float *prob = route_smem + (size_t)warp * experts;
     // A NaN or an infinity among the logits has no ranking (the reference's router refuses such a row:
     // "router produced invalid logits", src/nn/moe.rs:392-397): report it through the status word, give the token
     // the first `used` experts with weight zero so that everything downstream stays in range, and stop.
@@ -107,10 +123,8 @@ __device__ __forceinline__ void route_token(float *route_smem, const float *__re
         weights[(size_t)t * used + k] = norm ? v / picked_sum : v;
     }
     if (shared_gate) {
-        float dot = 0.f;
-        for (uint32_t i = lane; i < hidden; i += 32) dot = fmaf(x[(size_t)t * hidden + i], shared_w[i], dot);
-        dot = warp_sum(dot);
-        if (lane == 0) gate[t] = 1.f / (1.f + expf(-dot));
+        const float gv = fqk::route_gate(x + (size_t)t * hidden, shared_w, hidden, lane);
+        if (lane == 0) gate[t] = gv;
     } else if (lane == 0) {
         gate[t] = 1.f;
     }

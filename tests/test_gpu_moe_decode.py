@@ -1,0 +1,59 @@
+"""The one-launch MoE block of a single token against the kernels the block is otherwise made of (`moe_ffn_ep` on a
+communicator of one rank): the same bits, over shapes where its work is dealt out differently -- one and several
+superblocks per row, fewer and more tiles than SMs, every format pair it serves, a gate on the shared expert, sigmoid
+scores -- and what a router that yields no ranking leaves behind."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import ref
+
+pytestmark = pytest.mark.gpu
+
+
+def S():
+    from ferrum_b200 import surface
+    return surface
+
+
+def block(s, device, gu, dn, experts, used, hidden, ffn, shared, gate, sigmoid, seed=0):
+    M = lambda fmt, rows, cols, e, i: s.Matrix.from_packed(device, rows, cols, e, fmt, ref.random_matrix(fmt, rows * e, cols, seed + i))
+    w = torch.from_numpy((np.random.default_rng(seed).standard_normal(hidden) * 0.05).astype(np.float32)).cuda() if gate else None
+    return s.MoeFfn(M(ref.Q8_0, experts, hidden, 1, 1), M(gu, ffn, hidden, experts, 2), M(gu, ffn, hidden, experts, 3), M(dn, hidden, ffn, experts, 4),
+                    M(gu, shared, hidden, 1, 5), M(gu, shared, hidden, 1, 6), M(dn, hidden, shared, 1, 7), w, experts, used, hidden, ffn, shared,
+                    sigmoid, True)
+
+
+@pytest.mark.parametrize("gu,dn", [(ref.Q4_K, ref.Q6_K), (ref.Q4_K, ref.Q4_K), (ref.Q5_K, ref.Q6_K), (ref.Q5_K, ref.Q5_K), (ref.Q6_K, ref.Q6_K)])
+@pytest.mark.parametrize("experts,used,hidden,ffn,shared,gate,sigmoid", [
+    (16, 4, 512, 256, 256, False, False), (256, 8, 2048, 512, 512, True, False), (40, 12, 768, 768, 1024, True, True), (300, 1, 2560, 1280, 256, False, True)])
+def test_same_bits_as_the_chain_of_kernels(device, gu, dn, experts, used, hidden, ffn, shared, gate, sigmoid):
+    s = S()
+    f = block(s, device, gu, dn, experts, used, hidden, ffn, shared, gate, sigmoid)
+    n = s.moe_ffn_scratch_elems(device, f, 1)
+    comm = s.Comm(device, 0, 1, 4096 + used * hidden * 4)
+    for seed in range(3):
+        x = torch.from_numpy((np.random.default_rng(seed).standard_normal(hidden) * 0.12).astype(np.float32)).cuda()
+        one, chain = torch.zeros(hidden, device="cuda"), torch.zeros(hidden, device="cuda")
+        s.moe_ffn(device, f, x, 1, torch.zeros(n, device="cuda"), one)
+        s.moe_ffn_ep(device, comm, 4096, f, 0, x, 1, torch.zeros(n, device="cuda"), chain)
+        device.synchronize()
+        assert torch.equal(one, chain) and bool(torch.isfinite(one).all())
+    comm.close()
+
+
+def test_router_without_a_ranking_is_reported(device):
+    s = S()
+    f = block(s, device, ref.Q4_K, ref.Q6_K, 16, 4, 512, 256, 256, False, False)
+    x = torch.ones(512, device="cuda")
+    x[3] = float("inf")
+    n = s.moe_ffn_scratch_elems(device, f, 1)
+    out = torch.zeros(512, device="cuda")
+    s.moe_ffn(device, f, x, 1, torch.zeros(n, device="cuda"), out)
+    with pytest.raises(s.WeightError):
+        device.synchronize()
+    device.recover()
+    x[3] = 1.0
+    s.moe_ffn(device, f, x, 1, torch.zeros(n, device="cuda"), out)
+    device.synchronize()
+    assert bool(torch.isfinite(out).all())
