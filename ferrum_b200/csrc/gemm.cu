@@ -329,9 +329,11 @@ __device__ __forceinline__ void epilogue(uint32_t tmem, int warp, int lane, uint
 // store them.
 //
 // MODE 2 (dense, F32 callers): near-fp32 products from bf16 operands.  Both operands are split in two bf16
-// terms (v = hi + lo, lo = bf16(v - hi)) and every k-block is walked three times: hi x hi, hi x lo, lo x hi
-// (w_hi, w_hi, w_lo against x_hi, x_lo, x_hi); the caller lays X out as [m][3 * cols] in that order.  The
-// dropped lo x lo term and the residuals are 2^-17 of a product.
+// terms (v = hi + lo, lo = bf16(v - hi)) and every k-block is multiplied three times: w_hi x_hi, w_lo x_hi, w_hi x_lo.
+// Each of the four tiles is decoded or loaded once and stays for the products that use it (an A stage is the pair w_hi,
+// w_lo; the caller lays X out as [m][2 * cols], 64 hi then 64 lo per k-block).  The dropped lo x lo term and the residuals
+// are 2^-17 of a product.  (Walked as three k-blocks of their own, with w_hi decoded and x_hi loaded twice, and X so wide
+// that 512 rows of 17408 took two launches: a 27B-class layer of 512 rows 1468 -> 930 us.)
 // Up to four matrices of one format and width that share X (q|k|v, gate|up): their row tiles are counted
 // through, so one launch fills the machine where the small ones alone would not.
 struct GemmMany {
@@ -356,7 +358,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ 
     using SM = Smem<BN>;
     SM *sm = reinterpret_cast<SM *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t k_first = 0, k_iters = cols / BK * (PRECISE ? 3 : 1), n0, m0, m_end = m; // in units: (k-block, term)
+    constexpr uint32_t TERMS = PRECISE ? 2 : 1, A_RING = A_STAGES / TERMS; // tiles of an A stage; stages
+    uint32_t k_first = 0, k_iters = cols / BK, n0, m0, m_end = m;
     float *partial = nullptr;
     if (GROUPED) {
         // blockIdx.y counts activation tiles over all groups in order; `full_tiles` holds the group count.
@@ -421,7 +424,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ 
     const uint32_t nblk = cols / nblk_div;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < A_STAGES; s++) {
+        for (uint32_t s = 0; s < A_RING; s++) {
             mbar_init(&sm->full_a[s], PRODUCER_WARPS * 32);
             mbar_init(&sm->empty_a[s], 1);
         }
@@ -450,11 +453,11 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ 
             bool ok = true;
             for (uint32_t it = 0; it < k_iters && ok; it++) {
 #pragma unroll
-                for (int h = 0; h < NSUB; h++) {
-                    const uint32_t ib = it * NSUB + h, s = ib % B_SLOTS;
+                for (int h = 0; h < (int)(NSUB * TERMS); h++) { // rows of sub-tile h / TERMS, term h % TERMS
+                    const uint32_t ib = it * NSUB * TERMS + h, s = ib % B_SLOTS;
                     if (!(ok = mbar_wait(&sm->empty_b[s], ((ib / B_SLOTS) & 1) ^ 1, sm, status))) break;
                     mbar_expect_tx(&sm->full_b[s], b_bytes);
-                    tma_load_2d(sm->b[s], &xmap, (int)((k_first + it) * BK), (int)(m0 + h * MMA_N), &sm->full_b[s]);
+                    tma_load_2d(sm->b[s], &xmap, (int)(((k_first + it) * TERMS + h % TERMS) * BK), (int)(m0 + h / TERMS * MMA_N), &sm->full_b[s]);
                     issued = ib + 1;
                 }
             }
@@ -471,18 +474,23 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ 
         if (lane == 0) {
             bool ok = true;
             for (uint32_t it = 0; it < k_iters && ok; it++) {
-                const int sa = it % A_STAGES;
-                if (!mbar_wait(&sm->full_a[sa], (it / A_STAGES) & 1, sm, status)) break;
-                const uint64_t adesc = umma_desc(smem_u32(sm->a[sa]));
+                const uint32_t sa = it % A_RING;
+                if (!mbar_wait(&sm->full_a[sa], (it / A_RING) & 1, sm, status)) break;
+                const uint64_t adesc = umma_desc(smem_u32(sm->a[sa * TERMS]));
 #pragma unroll
-                for (int h = 0; h < NSUB; h++) { // each 256-row part of the activation tile has its own accumulator columns
-                    const uint32_t ib = it * NSUB + h, sb = ib % B_SLOTS;
+                for (int ht = 0; ht < (int)(NSUB * TERMS); ht++) { // each 256-row part of the activation tile has its own accumulator columns
+                    const uint32_t h = ht / TERMS, term = ht % TERMS, ib = it * NSUB * TERMS + ht, sb = ib % B_SLOTS;
                     if (!(ok = mbar_wait(&sm->full_b[sb], (ib / B_SLOTS) & 1, sm, status))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bdesc = umma_desc(smem_u32(sm->b[sb]));
 #pragma unroll
                     for (int k = 0; k < BK / 16; k++) // 16 bf16 = 32 bytes = 2 descriptor units along K
-                        umma_bf16(tmem + h * MMA_N, adesc + 2 * k, bdesc + 2 * k, IDESC, (it | k) != 0);
+                        umma_bf16(tmem + h * MMA_N, adesc + 2 * k, bdesc + 2 * k, IDESC, (it | term | k) != 0);
+                    if (PRECISE && term == 0) { // w_lo, the second tile of the stage
+                        const uint64_t lodesc = umma_desc(smem_u32(sm->a[sa * TERMS + TERMS - 1]));
+#pragma unroll
+                        for (int k = 0; k < BK / 16; k++) umma_bf16(tmem + h * MMA_N, lodesc + 2 * k, bdesc + 2 * k, IDESC, 1u);
+                    }
                     umma_commit(&sm->empty_b[sb]); // the slot is free once these MMAs have read it
                 }
                 if (ok) umma_commit(&sm->empty_a[sa]);
@@ -498,28 +506,32 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ 
         const uint32_t last = k_first + k_iters - 1;
         Raw<FMT> ring[PREFETCH];
 #pragma unroll
-        for (int j = 0; j < PREFETCH; j++) ring[j] = load_raw<FMT>(rowp, nblk, min(k_first + j, last) / (PRECISE ? 3 : 1), part);
+        for (int j = 0; j < PREFETCH; j++) ring[j] = load_raw<FMT>(rowp, nblk, min(k_first + j, last), part);
         bool go = true;
         for (uint32_t it0 = 0; it0 < k_iters && go; it0 += PREFETCH) {
 #pragma unroll
             for (int j = 0; j < PREFETCH; j++) {
                 const uint32_t it = it0 + j;
                 if (it >= k_iters) break;
-                const int s = it % A_STAGES;
-                uint32_t v[16];
+                const uint32_t s = it % A_RING;
+                uint32_t v[TERMS][16];
                 const uint32_t unit = k_first + it;
-                decode_raw<FMT>(ring[j], unit / (PRECISE ? 3 : 1), part, PRECISE && unit % 3 == 2, v);
-                ring[j] = load_raw<FMT>(rowp, nblk, min(unit + PREFETCH, last) / (PRECISE ? 3 : 1), part);
+#pragma unroll
+                for (uint32_t term = 0; term < TERMS; term++) decode_raw<FMT>(ring[j], unit, part, term == 1, v[term]);
+                ring[j] = load_raw<FMT>(rowp, nblk, min(unit + PREFETCH, last), part);
                 if (!live) {
 #pragma unroll
-                    for (int i = 0; i < 16; i++) v[i] = 0u;
+                    for (uint32_t i = 0; i < 16 * TERMS; i++) v[i / 16][i % 16] = 0u;
                 }
-                if (!mbar_wait(&sm->empty_a[s], ((it / A_STAGES) & 1) ^ 1, sm, status)) { go = false; break; }
-                uint8_t *tile_row = sm->a[s] + r * 128;
+                if (!mbar_wait(&sm->empty_a[s], ((it / A_RING) & 1) ^ 1, sm, status)) { go = false; break; }
 #pragma unroll
-                for (int c = 0; c < 4; c++) { // 16-byte chunk 4 part + c of the row, at its swizzled place
-                    const int chunk = (4 * part + c) ^ (r & 7);
-                    *reinterpret_cast<uint4 *>(tile_row + 16 * chunk) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                for (uint32_t term = 0; term < TERMS; term++) {
+                    uint8_t *tile_row = sm->a[s * TERMS + term] + r * 128;
+#pragma unroll
+                    for (int c = 0; c < 4; c++) { // 16-byte chunk 4 part + c of the row, at its swizzled place
+                        const int chunk = (4 * part + c) ^ (r & 7);
+                        *reinterpret_cast<uint4 *>(tile_row + 16 * chunk) = make_uint4(v[term][4 * c], v[term][4 * c + 1], v[term][4 * c + 2], v[term][4 * c + 3]);
+                    }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic-proxy stores -> tensor-core reads
                 mbar_arrive(&sm->full_a[s]);
@@ -571,19 +583,18 @@ __global__ void k_to_bf16(const float *__restrict__ x, __nv_bfloat16 *__restrict
     }
 }
 
-// X (fp32) as two bf16 terms laid out for MODE 2: k-block b of a row becomes the three 64-wide blocks
-// hi, lo, hi at 3 b, 3 b + 1, 3 b + 2, with hi = bf16(x) and lo = bf16(x - hi).
-__global__ void k_split3(const float *__restrict__ x, __nv_bfloat16 *__restrict__ out, uint32_t cols, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// X (fp32, `cols` a multiple of BK) as two bf16 terms laid out for MODE 2: k-block b of a row becomes the two 64-wide
+// blocks hi and lo at 2 b and 2 b + 1, with hi = bf16(x) and lo = bf16(x - hi).  Four values per thread.
+__global__ void __launch_bounds__(256) k_split2(const float *__restrict__ x, __nv_bfloat16 *__restrict__ out, uint32_t cols, size_t n) {
+    const size_t i = ((size_t)blockIdx.x * 256 + threadIdx.x) * 4;
     if (i >= n) return;
     const size_t row = i / cols;
-    const uint32_t k = (uint32_t)(i % cols), b = k / BK, j = k % BK;
-    const float v = x[i];
-    const __nv_bfloat16 hi = __float2bfloat16_rn(v), lo = __float2bfloat16_rn(v - __bfloat162float(hi));
-    __nv_bfloat16 *dst = out + row * (size_t)cols * 3 + (size_t)b * 3 * BK + j;
-    dst[0] = hi;
-    dst[BK] = lo;
-    dst[2 * BK] = hi;
+    const uint32_t k = (uint32_t)(i - row * cols), b = k / BK, j = k % BK;
+    const float4 v = *reinterpret_cast<const float4 *>(x + i);
+    const uint32_t h0 = pack_bf16(v.x, v.y), h1 = pack_bf16(v.z, v.w);
+    __nv_bfloat16 *dst = out + row * (size_t)cols * 2 + (size_t)b * 2 * BK + j;
+    *reinterpret_cast<uint2 *>(dst) = make_uint2(h0, h1);
+    *reinterpret_cast<uint2 *>(dst + BK) = make_uint2(pack_term(v.x, v.y, true), pack_term(v.z, v.w, true));
 }
 
 // The tiles that were split along K: their fp32 partial sums added in split order (deterministic), rounded and
@@ -630,7 +641,7 @@ int launch(fq_device *dev, const ProjectArgs &a, const CUtensorMap &map, uint32_
         if (e != cudaSuccess) return fq_check_cuda(dev, e, "gemm shared memory");
         configured = true;
     }
-    const uint32_t tiles_x = many.count > 1 ? many.tx_end[many.count - 1] : (a.rows + BM - 1) / BM, k_iters = a.cols / BK * (MODE == 2 ? 3 : 1);
+    const uint32_t tiles_x = many.count > 1 ? many.tx_end[many.count - 1] : (a.rows + BM - 1) / BM, k_iters = a.cols / BK;
     if (GROUPED) {
         // At most one partly filled tile per group on top of the full ones (m_rows = all groups' rows).
         const uint32_t per_group = (a.max_rows + BN - 1) / BN;
@@ -642,13 +653,14 @@ int launch(fq_device *dev, const ProjectArgs &a, const CUtensorMap &map, uint32_
         return FQ_OK;
     }
     // Whole waves of tiles run one tile per block.  A remainder that would fill less than three quarters of a
-    // wave is split along K into about one block per SM, each with at least 8 k-blocks and a workspace slot.
+    // wave is split along K into about one block per SM, each with at least 8 k-blocks' products (MODE 2: three a
+    // k-block) and a workspace slot.
     const uint32_t tiles = tiles_x * ((m_rows + BN - 1) / BN), sms = (uint32_t)dev->sm_count;
     const uint32_t rest = tiles % sms;
     uint32_t full = tiles, splits = 1, per = k_iters;
     if (rest && rest * 4 < sms * 3) {
         const uint32_t cap = (uint32_t)std::min<size_t>(sms / rest, dev->gemm_ws_bytes / ((size_t)rest * BN * BM * sizeof(float)));
-        const uint32_t want = std::min({cap, std::max(1u, k_iters / 8), 16u});
+        const uint32_t want = std::min({cap, std::max(1u, k_iters / (MODE == 2 ? 3 : 8)), 16u});
         if (want > 1) {
             per = (k_iters + want - 1) / want;
             splits = (k_iters + per - 1) / per; // no split is left without work
@@ -1274,18 +1286,18 @@ int fq_launch_gemm_tc(fq_device *dev, const ProjectArgs &a) {
         if (rc != FQ_OK) return rc;
         return fq_end_enqueue(dev, "gemm_tc", 1);
     }
-    const size_t half = dev->xprep_bytes / 2, row_bytes3 = (size_t)a.cols * 3 * sizeof(__nv_bfloat16);
-    uint32_t slice = (uint32_t)std::min<size_t>(a.m, half / row_bytes3);
+    const size_t half = dev->xprep_bytes / 2, row_bytes2 = (size_t)a.cols * 2 * sizeof(__nv_bfloat16);
+    uint32_t slice = (uint32_t)std::min<size_t>(a.m, half / row_bytes2);
     if (slice < a.m) slice = slice >= 512 ? (slice & ~511u) : (slice & ~255u); // whole tiles per slice
     if (slice == 0) return FQ_ERR_UNSUPPORTED;
     int kernels = 0;
     for (uint32_t m0 = 0; m0 < a.m; m0 += slice) {
         const uint32_t mm = std::min(slice, a.m - m0);
         dev->xprep_turn ^= 1u;
-        __nv_bfloat16 *x3 = (__nv_bfloat16 *)((uint8_t *)dev->xprep + (dev->xprep_turn ? half : 0));
+        __nv_bfloat16 *x2 = (__nv_bfloat16 *)((uint8_t *)dev->xprep + (dev->xprep_turn ? half : 0));
         const size_t n = (size_t)mm * a.cols;
-        k_split3<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>((const float *)a.x + (size_t)m0 * a.cols, x3, a.cols, n);
-        if (int rc = make_map(dev, &map, x3, a.cols * 3, mm, 256, &b_bytes)) return rc;
+        k_split2<<<(unsigned)((n + 1023) / 1024), 256, 0, dev->stream>>>((const float *)a.x + (size_t)m0 * a.cols, x2, a.cols, n);
+        if (int rc = make_map(dev, &map, x2, a.cols * 2, mm, 256, &b_bytes)) return rc;
         ProjectArgs s = a;
         s.m = mm;
         s.y = (float *)a.y + (size_t)m0 * a.rows;
@@ -1307,7 +1319,7 @@ int fq_launch_gemm_tc_many(fq_device *dev, const ProjectArgs *a, uint32_t count)
     if (f.format != FQ_Q4_K && f.format != FQ_Q5_K && f.format != FQ_Q6_K && f.format != FQ_Q8_0) return FQ_ERR_UNSUPPORTED;
     if (f.format == FQ_Q4_K && (f.row_bytes % 16)) return FQ_ERR_UNSUPPORTED;
     if (f.m <= (uint32_t)FQ_GEMV_MAX_M) return FQ_ERR_UNSUPPORTED;
-    if (wide && (size_t)f.m * f.cols * 3 * sizeof(__nv_bfloat16) > dev->xprep_bytes / 2) return FQ_ERR_UNSUPPORTED;
+    if (wide && (size_t)f.m * f.cols * 2 * sizeof(__nv_bfloat16) > dev->xprep_bytes / 2) return FQ_ERR_UNSUPPORTED;
     GemmMany many{};
     many.count = count;
     uint32_t tx = 0;
@@ -1325,10 +1337,10 @@ int fq_launch_gemm_tc_many(fq_device *dev, const ProjectArgs *a, uint32_t count)
     uint32_t b_bytes = 0;
     if (wide) {
         dev->xprep_turn ^= 1u;
-        __nv_bfloat16 *x3 = (__nv_bfloat16 *)((uint8_t *)dev->xprep + (dev->xprep_turn ? dev->xprep_bytes / 2 : 0));
+        __nv_bfloat16 *x2 = (__nv_bfloat16 *)((uint8_t *)dev->xprep + (dev->xprep_turn ? dev->xprep_bytes / 2 : 0));
         const size_t n = (size_t)f.m * f.cols;
-        k_split3<<<(unsigned)((n + 255) / 256), 256, 0, dev->stream>>>((const float *)f.x, x3, f.cols, n);
-        if (int rc = make_map(dev, &map, x3, f.cols * 3, f.m, 256, &b_bytes)) return rc;
+        k_split2<<<(unsigned)((n + 1023) / 1024), 256, 0, dev->stream>>>((const float *)f.x, x2, f.cols, n);
+        if (int rc = make_map(dev, &map, x2, f.cols * 2, f.m, 256, &b_bytes)) return rc;
         const int rc = f.m >= 384 ? launch_fmt<512, float, 2>(dev, f, map, b_bytes, f.m, many) : launch_fmt<256, float, 2>(dev, f, map, b_bytes, f.m, many);
         if (rc != FQ_OK) return rc;
         return fq_end_enqueue(dev, "gemm_tc", 2);
