@@ -108,6 +108,15 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
                  : "memory");
 }
 
+// One lane of a converged warp.  The branches that issue TMA and MMA instructions are taken by it, not by `lane == 0`: the
+// compiler then knows that a single thread runs them and feeds their uniform operands without a loop over lanes (four
+// prompt projections of 2048 rows 1437 -> 1290 us).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
+}
+
 // Shared-memory operand descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
@@ -448,7 +457,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ 
     const uint32_t tmem = *(volatile uint32_t *)&sm->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t issued = 0;
             bool ok = true;
             for (uint32_t it = 0; it < k_iters && ok; it++) {
@@ -471,7 +480,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap xmap, const uint8_t *__restrict__ 
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             for (uint32_t it = 0; it < k_iters && ok; it++) {
                 const uint32_t sa = it % A_RING;
@@ -1000,7 +1009,7 @@ k_gemm_f16g(const __grid_constant__ GMaps M, const __grid_constant__ GJob J) {
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t ix = 0;
             bool ok = true;
             for (uint32_t i = 0; i < my_items && ok; i++) {
@@ -1024,7 +1033,7 @@ k_gemm_f16g(const __grid_constant__ GMaps M, const __grid_constant__ GJob J) {
                     for (uint32_t n = 0; n < WAIT_LIMIT && !mbar_try(&sm->full_x[u % GRaw<FMT>::X_SLOTS], (u / GRaw<FMT>::X_SLOTS) & 1); n++) {}
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it_n = 0;
             bool ok = true;
             for (uint32_t i = 0; i < my_items && ok; i++) {
@@ -1051,7 +1060,7 @@ k_gemm_f16g(const __grid_constant__ GMaps M, const __grid_constant__ GJob J) {
         // the ring holds.  The decoding threads so have no loads of their own in flight (their
         // proxy fence would wait for them), and the copies do not queue behind the SM's load unit.
         if constexpr (FMT == FQ_Q4_K) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr int RAW = GRaw<FMT>::STAGES;
             uint32_t ir = 0;
             bool ok = true;
