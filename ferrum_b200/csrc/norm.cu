@@ -6,6 +6,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <utility>
 
 #include "gemv_common.cuh"
 #include "internal.h"
@@ -92,6 +93,9 @@ k_argmax(const float *__restrict__ x, uint32_t n, uint32_t *__restrict__ out) {
     __shared__ uint32_t best_i[16];
     __shared__ float part_v[ARGMAX_CLUSTER];
     __shared__ uint32_t part_i[ARGMAX_CLUSTER];
+    // Block 0's shared memory may be written once every block of the cluster is known to run: arrived here, waited for
+    // just before the first remote store, so that the scan of the row hides it.
+    cg::cluster_group::arrival_token running = cluster.barrier_arrive();
     pdl_trigger();
     pdl_wait(); // the logits are the output of the kernel before
     const uint32_t tid = threadIdx.x, rank = cluster.block_rank();
@@ -127,6 +131,7 @@ k_argmax(const float *__restrict__ x, uint32_t n, uint32_t *__restrict__ out) {
         best_i[tid >> 5] = bi;
     }
     __syncthreads();
+    cluster.barrier_wait(std::move(running));
     if (tid < 32) {
         bv = best_v[tid & 15];
         bi = best_i[tid & 15];
