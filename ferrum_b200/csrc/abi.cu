@@ -1163,6 +1163,8 @@ extern "C" int fq_moe_ffn(fq_device *dev, const fq_moe_ffn_desc *f, const float 
         f->up_exps->expert_rows() != ef || f->down_exps->experts != experts || f->down_exps->expert_rows() != hidden ||
         f->down_exps->cols != ef || f->shared_gate->rows != f->shared_ffn || f->shared_down->rows != hidden)
         return fq_fail(dev, FQ_ERR_SHAPE, "MoE matrices do not match the description");
+    for (const fq_matrix *w : {f->router, f->gate_exps, f->up_exps, f->down_exps, f->shared_gate, f->shared_up, f->shared_down})
+        if (w->dev != dev) return fq_fail(dev, FQ_ERR_DEVICE, "matrix belongs to another device handle");
     MoeScratch s = moe_layout(f, m, scratch);
     if (scratch_elems < s.total) return fq_fail(dev, FQ_ERR_SHAPE, "MoE scratch holds %zu of %zu floats", scratch_elems, s.total);
     const size_t routes = m * used;

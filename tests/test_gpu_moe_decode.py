@@ -57,3 +57,18 @@ def test_router_without_a_ranking_is_reported(device):
     s.moe_ffn(device, f, x, 1, torch.zeros(n, device="cuda"), out)
     device.synchronize()
     assert bool(torch.isfinite(out).all())
+
+
+@pytest.mark.parametrize("m", [1, 2, 21])
+@pytest.mark.parametrize("which", ["router", "gate_exps", "up_exps", "down_exps", "shared_gate", "shared_up", "shared_down"])
+def test_matrix_of_another_handle_is_refused(device, which, m):
+    s = S()
+    other = s.Device(0)
+    f = block(s, device, ref.Q4_K, ref.Q6_K, 16, 4, 512, 256, 256, False, False)
+    g = block(s, other, ref.Q4_K, ref.Q6_K, 16, 4, 512, 256, 256, False, False)
+    scratch = torch.zeros(s.moe_ffn_scratch_elems(device, f, m), device="cuda")
+    setattr(f, which, getattr(g, which))
+    before = device.counters().dispatches
+    with pytest.raises(s.DeviceMismatch):
+        s.moe_ffn(device, f, torch.zeros(m * 512, device="cuda"), m, scratch, torch.zeros(m * 512, device="cuda"))
+    assert device.counters().dispatches == before  # nothing was enqueued
