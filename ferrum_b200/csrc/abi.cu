@@ -1168,17 +1168,12 @@ extern "C" int fq_moe_ffn(fq_device *dev, const fq_moe_ffn_desc *f, const float 
     MoeScratch s = moe_layout(f, m, scratch);
     if (scratch_elems < s.total) return fq_fail(dev, FQ_ERR_SHAPE, "MoE scratch holds %zu of %zu floats", scratch_elems, s.total);
     const size_t routes = m * used;
-    if (m == 1 && !dev->exact) {
-        // One token: the whole block is one launch where the shapes have it.
-        if (int rc = fq_begin_enqueue(dev)) return rc;
-        if (int rc = fq_check_binding(dev, x, hidden * 4, "x")) return rc;
-        if (int rc = fq_check_binding(dev, scratch, s.total * 4, "scratch")) return rc;
-        if (int rc = fq_check_binding(dev, out, hidden * 4, "out")) return rc;
-        if (f->shared_gate_inp)
-            if (int rc = fq_check_binding(dev, f->shared_gate_inp, hidden * 4, "shared gate weight")) return rc;
-        if (int rc = fq_check_no_alias(dev, scratch, s.total * 4, x, hidden * 4, "scratch")) return rc;
-        const int rc = fq_launch_moe_decode(dev, f, x, s.logits, s.g, s.u, s.shared_tmp, s.shared_tmp + f->shared_ffn, out);
-        if (rc == FQ_OK) fq_note_write(dev, out, hidden * 4);
+    // One token: the whole block is one launch where the shapes have it.  Its blocks read x, the gate's weight and the
+    // scratch at different times, so where one of these or the output overlaps the scratch the chain of kernels below
+    // runs, with its own checks.
+    auto in_scratch = [&](const float *p, size_t n) { return p && p < scratch + s.total && scratch < p + n; };
+    if (m == 1 && !dev->exact && !in_scratch(x, hidden) && !in_scratch(out, hidden) && !in_scratch(f->shared_gate_inp, hidden)) {
+        const int rc = fq_launch_moe_decode(dev, f, x, scratch, s.total, s.logits, s.g, s.u, s.shared_tmp, s.shared_tmp + f->shared_ffn, out);
         if (rc != FQ_ERR_UNSUPPORTED) return rc;
     }
     const bool identity = routes <= MV_ID_MAX_ROUTES || dev->exact;

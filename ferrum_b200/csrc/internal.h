@@ -189,8 +189,8 @@ int fq_moe_route_map(fq_device *dev, const float *logits, const float *x, const 
                      uint32_t hidden, uint32_t tokens, int sigmoid, int norm, int shared_gate, uint32_t *ids, float *weights, float *gate,
                      uint32_t *offsets, uint32_t *sorted, uint32_t *position);
 // The MoE block of one token in one launch (moe_decode.cu); FQ_ERR_UNSUPPORTED when the shapes or formats have none.
-int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *x, float *logits, float *g, float *u, float *shared_g, float *shared_u,
-                         float *out);
+int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *x, float *scratch, size_t scratch_elems, float *logits, float *g, float *u,
+                         float *shared_g, float *shared_u, float *out);
 int fq_launch_glu_bf16(fq_device *dev, const float *gate, const float *up, size_t n, const uint32_t *range, uint32_t stride, uint32_t width,
                        void *out);
 // out[row] = expert of expert-sorted row `row` minus `first`, or an id that names no expert when it is not one

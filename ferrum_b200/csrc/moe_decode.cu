@@ -325,9 +325,10 @@ template <int GU, int DN> cudaError_t launch(fq_device *dev, const MoeDecodeJob 
 
 // One token on the shapes and formats above (the experts' and the shared expert's matrices of one format per role, a
 // Q8_0 router, widths a whole number of superblocks); FQ_ERR_UNSUPPORTED otherwise, nothing enqueued.  `logits` ..
-// `shared_u`: scratch of experts, used * ffn (twice) and shared_ffn (twice) floats.
-int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *x, float *logits, float *g, float *u, float *shared_g, float *shared_u,
-                         float *out) {
+// `shared_u`: parts of `scratch`, of experts, used * ffn (twice) and shared_ffn (twice) floats; x, out and the gate's
+// weight lie outside `scratch`.
+int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *x, float *scratch, size_t scratch_elems, float *logits, float *g, float *u,
+                         float *shared_g, float *shared_u, float *out) {
     const int gu = f->gate_exps->format, dn = f->down_exps->format;
     const uint32_t H = f->hidden, F = f->expert_ffn, SF = f->shared_ffn;
     if (f->router->format != FQ_Q8_0 || f->up_exps->format != gu || f->shared_gate->format != gu || f->shared_up->format != gu || f->shared_down->format != dn)
@@ -372,13 +373,21 @@ int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *
     J.status = dev->status_dev;
     const size_t smem = moe_decode_smem(H, F, SF, f->used).total;
     if (smem > 200 * 1024) return FQ_ERR_UNSUPPORTED;
-    cudaError_t e;
-    if (gu == FQ_Q4_K && dn == FQ_Q6_K) e = launch<FQ_Q4_K, FQ_Q6_K>(dev, J, smem);
-    else if (gu == FQ_Q4_K && dn == FQ_Q4_K) e = launch<FQ_Q4_K, FQ_Q4_K>(dev, J, smem);
-    else if (gu == FQ_Q5_K && dn == FQ_Q6_K) e = launch<FQ_Q5_K, FQ_Q6_K>(dev, J, smem);
-    else if (gu == FQ_Q5_K && dn == FQ_Q5_K) e = launch<FQ_Q5_K, FQ_Q5_K>(dev, J, smem);
-    else if (gu == FQ_Q6_K && dn == FQ_Q6_K) e = launch<FQ_Q6_K, FQ_Q6_K>(dev, J, smem);
-    else return FQ_ERR_UNSUPPORTED;
-    if (int rc = fq_check_cuda(dev, e, "moe decode launch")) return rc;
+    auto kernel = gu == FQ_Q4_K && dn == FQ_Q6_K   ? launch<FQ_Q4_K, FQ_Q6_K>
+                  : gu == FQ_Q4_K && dn == FQ_Q4_K ? launch<FQ_Q4_K, FQ_Q4_K>
+                  : gu == FQ_Q5_K && dn == FQ_Q6_K ? launch<FQ_Q5_K, FQ_Q6_K>
+                  : gu == FQ_Q5_K && dn == FQ_Q5_K ? launch<FQ_Q5_K, FQ_Q5_K>
+                  : gu == FQ_Q6_K && dn == FQ_Q6_K ? launch<FQ_Q6_K, FQ_Q6_K>
+                                                   : nullptr;
+    if (!kernel) return FQ_ERR_UNSUPPORTED;
+    if (int rc = fq_begin_enqueue(dev)) return rc;
+    if (int rc = fq_check_binding(dev, x, (size_t)H * 4, "x")) return rc;
+    if (int rc = fq_check_binding(dev, scratch, scratch_elems * 4, "scratch")) return rc;
+    if (int rc = fq_check_binding(dev, out, (size_t)H * 4, "out")) return rc;
+    if (f->shared_gate_inp)
+        if (int rc = fq_check_binding(dev, f->shared_gate_inp, (size_t)H * 4, "shared gate weight")) return rc;
+    if (int rc = fq_check_no_alias(dev, scratch, scratch_elems * 4, x, (size_t)H * 4, "scratch")) return rc;
+    if (int rc = fq_check_cuda(dev, kernel(dev, J, smem), "moe decode launch")) return rc;
+    fq_note_write(dev, out, (size_t)H * 4);
     return fq_end_enqueue(dev, "moe_decode", 1);
 }

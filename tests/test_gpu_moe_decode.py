@@ -72,3 +72,26 @@ def test_matrix_of_another_handle_is_refused(device, which, m):
     with pytest.raises(s.DeviceMismatch):
         s.moe_ffn(device, f, torch.zeros(m * 512, device="cuda"), m, scratch, torch.zeros(m * 512, device="cuda"))
     assert device.counters().dispatches == before  # nothing was enqueued
+
+
+@pytest.mark.parametrize("inside", ["x", "out", "x and out"])
+def test_operands_inside_the_scratch(device, inside):
+    """One token with x or the output in a part of the scratch that the block does not use at this width (the gathered
+    rows, which lie before four index arrays at its end): taken, and the same bits as with buffers of their own."""
+    s = S()
+    experts, used, hidden = 16, 4, 512
+    f = block(s, device, ref.Q4_K, ref.Q6_K, experts, used, hidden, 256, 256, True, False)
+    n = s.moe_ffn_scratch_elems(device, f, 1)
+    x = torch.from_numpy((np.random.default_rng(5).standard_normal(hidden) * 0.12).astype(np.float32)).cuda()
+    want, out = torch.zeros(hidden, device="cuda"), torch.zeros(hidden, device="cuda")
+    s.moe_ffn(device, f, x, 1, torch.zeros(n, device="cuda"), want)
+    scratch = torch.zeros(n, device="cuda")
+    at = n - (3 * used + (experts + 1 + 3) // 4 * 4) - used * hidden
+    if "x" in inside:
+        scratch[at:at + hidden] = x
+        x = scratch[at:at + hidden]
+    if "out" in inside:
+        out = scratch[at + hidden:at + 2 * hidden]
+    s.moe_ffn(device, f, x, 1, scratch, out)
+    device.synchronize()
+    assert torch.equal(out, want) and bool(want.abs().max() > 0)
