@@ -502,15 +502,15 @@ template <typename... Args> void launch_combine(cudaStream_t stream, const float
 // out = g / (1 + exp(-g)) * u, four values per thread (the remainder one by one)
 __device__ __forceinline__ float swiglu(float x, float u) { return x / (1.f + expf(-x)) * u; }
 __global__ void __launch_bounds__(256)
-k_swiglu(const float *__restrict__ g, const float *__restrict__ u, size_t n, float *__restrict__ y) {
+k_swiglu(const float *g, const float *u, size_t n, float *y) {
     fqk::pdl_trigger();
-    fqk::pdl_wait();
+    fqk::pdl_wait(); // g and u are the outputs of kernels that may still run when this grid starts: coherent loads
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i + 4 <= n) {
-        const float4 a = *reinterpret_cast<const float4 *>(g + i), b = *reinterpret_cast<const float4 *>(u + i);
+        const float4 a = __ldcg(reinterpret_cast<const float4 *>(g + i)), b = __ldcg(reinterpret_cast<const float4 *>(u + i));
         *reinterpret_cast<float4 *>(y + i) = make_float4(swiglu(a.x, b.x), swiglu(a.y, b.y), swiglu(a.z, b.z), swiglu(a.w, b.w));
     } else {
-        for (size_t j = i; j < n; j++) y[j] = swiglu(g[j], u[j]);
+        for (size_t j = i; j < n; j++) y[j] = swiglu(__ldcg(g + j), __ldcg(u + j));
     }
 }
 

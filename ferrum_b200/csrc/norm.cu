@@ -19,10 +19,12 @@ using namespace fqk;
 // before it.  A decode step's row is latency-bound: 17-22 us with one warp walking the row, about 3 us so.
 constexpr int NORM_CACHED = 8; // float4s a thread keeps
 __global__ void __launch_bounds__(NORM_WARPS * 32)
-k_rmsnorm(const float *__restrict__ x, const float *__restrict__ r, const float *__restrict__ w, uint32_t n, float eps, float *__restrict__ h,
-          float *__restrict__ y) {
+k_rmsnorm(const float *x, const float *r, const float *__restrict__ w, uint32_t n, float eps, float *h, float *y) {
     pdl_trigger();
-    pdl_wait(); // x and r are the outputs of kernels before this one
+    // x and r are the outputs of kernels that may still run when this grid starts: coherent loads after the wait.  h may be
+    // x, and y may be x or r: every value of a row is read before the first of its y is written, and a value's h by the
+    // thread that read it.
+    pdl_wait();
     __shared__ float part[NORM_WARPS];
     constexpr uint32_t T = NORM_WARPS * 32;
     const uint32_t tid = threadIdx.x, n4 = n / 4;
@@ -35,13 +37,13 @@ k_rmsnorm(const float *__restrict__ x, const float *__restrict__ r, const float 
 #pragma unroll
     for (int j = 0; j < NORM_CACHED; j++) {
         const uint32_t i = tid + T * j;
-        if (i < n4) v[j] = xr[i];
+        if (i < n4) v[j] = __ldcg(xr + i);
     }
     if (r) { // h = x + r first; the norm is taken of h
 #pragma unroll
         for (int j = 0; j < NORM_CACHED; j++) {
             const uint32_t i = tid + T * j;
-            if (i < n4) v[j] = sum(v[j], rr[i]);
+            if (i < n4) v[j] = sum(v[j], __ldcg(rr + i));
         }
     }
     float ss = 0.f;
@@ -54,8 +56,8 @@ k_rmsnorm(const float *__restrict__ x, const float *__restrict__ r, const float 
         }
     }
     for (uint32_t i = tid + T * NORM_CACHED; i < n4; i += T) {
-        float4 a = xr[i];
-        if (r) hr[i] = a = sum(a, rr[i]);
+        float4 a = __ldcg(xr + i);
+        if (r) hr[i] = a = sum(a, __ldcg(rr + i));
         ss = norm_square(ss, a);
     }
     ss = norm_butterfly(ss);
@@ -70,7 +72,7 @@ k_rmsnorm(const float *__restrict__ x, const float *__restrict__ r, const float 
         const uint32_t i = tid + T * j;
         if (i < n4) yr[i] = scaled(v[j], g[i]);
     }
-    for (uint32_t i = tid + T * NORM_CACHED; i < n4; i += T) yr[i] = scaled(r ? hr[i] : xr[i], g[i]);
+    for (uint32_t i = tid + T * NORM_CACHED; i < n4; i += T) yr[i] = scaled(__ldcg((r ? hr : xr) + i), g[i]);
 }
 
 __device__ __forceinline__ void better(float &bv, uint32_t &bi, float ov, uint32_t oi) {
@@ -86,7 +88,7 @@ __device__ __forceinline__ void better(float &bv, uint32_t &bi, float ov, uint32
 constexpr int ARGMAX_CLUSTER = 8;
 template <int VEC>
 __global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(512)
-k_argmax(const float *__restrict__ x, uint32_t n, uint32_t *__restrict__ out) {
+k_argmax(const float *x, uint32_t n, uint32_t *out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ float best_v[16];
@@ -97,7 +99,7 @@ k_argmax(const float *__restrict__ x, uint32_t n, uint32_t *__restrict__ out) {
     // just before the first remote store, so that the scan of the row hides it.
     cg::cluster_group::arrival_token running = cluster.barrier_arrive();
     pdl_trigger();
-    pdl_wait(); // the logits are the output of the kernel before
+    pdl_wait(); // the logits are the output of a kernel that may still run when this grid starts: coherent loads from here on
     const uint32_t tid = threadIdx.x, rank = cluster.block_rank();
     x += (size_t)blockIdx.y * n;
     const uint32_t groups = (n + VEC - 1) / VEC, per = (groups + ARGMAX_CLUSTER - 1) / ARGMAX_CLUSTER;
@@ -113,13 +115,13 @@ k_argmax(const float *__restrict__ x, uint32_t n, uint32_t *__restrict__ out) {
 #pragma unroll 4
     for (uint32_t i = rank * per + tid; i < end; i += 512) {
         if constexpr (VEC == 4) {
-            const float4 v = reinterpret_cast<const float4 *>(x)[i];
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(x) + i);
             take(v.x, 4 * i);
             take(v.y, 4 * i + 1);
             take(v.z, 4 * i + 2);
             take(v.w, 4 * i + 3);
         } else {
-            take(x[i], i);
+            take(__ldcg(x + i), i);
         }
     }
     auto reduce = [&](int lanes) {
