@@ -18,7 +18,7 @@
 namespace {
 
 constexpr int WARPS = 8;
-constexpr uint32_t MAX_COLS_IQ4 = 65536; // 2 planes x cols bytes of shared memory
+constexpr uint32_t MAX_COLS_IQ4 = 16384; // wider rows run on the exact fp32 kernel
 
 // Shared memory: hi[cols], lo[cols] (signed bytes), isc[cols / 32] (1 / s).
 template <int FMT>
