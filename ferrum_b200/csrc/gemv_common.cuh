@@ -97,42 +97,54 @@ __device__ __forceinline__ int byte_s(uint32_t w, int i) {
 }
 __device__ __forceinline__ uint32_t word_of(const uint4 &v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
-// Eight activations of one lane as 24-bit integers x' = round(x * s) = 65536 hi + 256 mid + lo, all three signed bytes, s
-// the largest power of two with max|x| * s <= 8355711 over the superblock: what fp32 holds of the largest value and at
-// least 2^-24 of it for the others.  Non-finite superblocks as in Quant8 below.
+// Eight activations of one lane as 31-bit integers x' = round(x * 2^e) in four signed base-256 digits, p[0] the most
+// significant, 2^e the largest power of two with max|x| * 2^e <= 0x7F7F7F00 over the superblock, up to 2^149: a step is at
+// most 2^-30 of the superblock's largest value, and never more than fp32's own smallest, so less is dropped than the
+// products and sums of an fp32 dot product round off (24 bits of the largest value were not enough: 1.3 to 7 times the
+// error of the fp32 kernels on rows of 1024..2304 values, more where a superblock has an outlier).
+// inv = 2^-e.  A superblock with an infinity and no NaN: inv = +infinity and p[0] holds the sign (+-1) of every infinity,
+// 0 for the rest; with a NaN: inv is NaN.
 struct Quant8Wide {
-    uint8_t hi[8], mid[8], lo[8];
-    int e;
-    bool finite;
+    uint32_t p[4][2]; // values 0-3 and 4-7, one per byte
+    float inv;
 };
 __device__ __forceinline__ Quant8Wide quantize8_wide(const float (&v)[8]) {
     Quant8Wide q;
     float amax = 0.f;
-    bool bad = false;
+    bool nan = false;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        amax = fmaxf(amax, fabsf(v[i]));
-        bad |= !(fabsf(v[i]) < INFINITY);
+        amax = fmaxf(amax, fabsf(v[i])); // drops a NaN
+        nan |= v[i] != v[i];
     }
-    q.finite = __ballot_sync(0xffffffffu, bad) == 0u;
+    nan = __any_sync(0xffffffffu, nan);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    const bool finite = amax < INFINITY && !nan;
+    // amax = 1.f * 2^ex: e = 30 - ex, one less where the mantissa is above that of 0x7F7F7F00; a subnormal amax ends at 149.
+    const uint32_t bits = __float_as_uint(amax);
     int e = 0;
-    if (amax > 0.f && q.finite) {
-        int ex;
-        frexpf(amax, &ex);
-        e = max(-110, min(110, 23 - ex));
-        if (ldexpf(amax, e) > 8355711.f) e -= 1;
-    }
-    q.e = e;
-    const float s = ldexpf(1.f, e);
+    if (amax > 0.f && finite) e = min(149, 157 - (int)(bits >> 23) - ((bits & 0x7FFFFFu) > 0x7EFEFEu));
+    q.inv = e > 126 ? __uint_as_float(1u << (149 - e)) : __uint_as_float((uint32_t)(127 - e) << 23);
+    if (!finite) q.inv = nan ? __int_as_float(0x7fc00000) : INFINITY;
+    // 2^e may be beyond fp32: two factors.
+    const int e0 = e >> 1;
+    const float s0 = __uint_as_float((uint32_t)(127 + e0) << 23), s1 = __uint_as_float((uint32_t)(127 + e - e0) << 23);
+    uint32_t d[8]; // the digits of a value, the most significant in the top byte: adding 0x80 to every digit makes them unsigned
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int x = q.finite ? __float2int_rn(fminf(fmaxf(v[i] * s, -8355711.f), 8355711.f)) : 0;
-        const int m = (x + 128) >> 8, h = (m + 128) >> 8;
-        q.lo[i] = (uint8_t)(x - (m << 8));
-        q.mid[i] = (uint8_t)(m - (h << 8));
-        q.hi[i] = (uint8_t)h;
+    for (int i = 0; i < 8; i++) d[i] = ((uint32_t)__float2int_rn(v[i] * s0 * s1) + 0x80808080u) ^ 0x80808080u;
+    if (!finite)
+#pragma unroll
+        for (int i = 0; i < 8; i++) d[i] = nan || fabsf(v[i]) < INFINITY ? 0u : v[i] > 0.f ? 0x01000000u : 0xFF000000u;
+#pragma unroll
+    for (int h = 0; h < 2; h++) { // bytes of four values -> one word per digit
+        const uint32_t *x = d + 4 * h;
+        const uint32_t low01 = __byte_perm(x[0], x[1], 0x5140), low23 = __byte_perm(x[2], x[3], 0x5140);
+        const uint32_t top01 = __byte_perm(x[0], x[1], 0x7362), top23 = __byte_perm(x[2], x[3], 0x7362);
+        q.p[3][h] = __byte_perm(low01, low23, 0x5410);
+        q.p[2][h] = __byte_perm(low01, low23, 0x7632);
+        q.p[1][h] = __byte_perm(top01, top23, 0x5410);
+        q.p[0][h] = __byte_perm(top01, top23, 0x7632);
     }
     return q;
 }

@@ -1,4 +1,4 @@
-// Verify-width projections (2..16 activation rows) and grouped expert projections with few rows per expert,
+// Verify-width projections (2..16 activation rows; of the IQ4 formats from one) and grouped expert projections with few rows per expert,
 // on the integer tensor path with the ACTIVATION ROWS ON THE MMA's N SIDE (F32 in, F32 out).  The reference's
 // `h_mvb_*` / `h_mms_*` (src/metal/shaders/hybrid.metal:1330-1394, 1419-1495; dispatch
 // src/hybrid/engine.rs:3438-3460) and, over expert-sorted rows, `h_mm_id_*` (hybrid.metal:2430-2523).
@@ -10,12 +10,12 @@
 //                           (two shifts and two LOP3 per four weights; the factor 4 goes into d);
 //   B (k x 8 rows of x)     the activations as 16-bit integers x' = round(x * s) = 256 hi + lo, both halves
 //                           signed bytes, s a power of two per (row, superblock): two MMAs (hi, lo) on the same A;
-//                           The IQ4 formats: codebook values as s8, and x' of 24 bits (three planes, three MMAs);
+//                           The IQ4 formats: codebook values as s8, and x' of 31 bits (four planes, four MMAs);
 //   per scale group         acc_hi += scale * c_hi, acc_lo += scale * c_lo in integers (and, Q4_K, the minimums
 //                           times the activation sums); once per superblock one conversion and FMA with d / s.
 //
-// The result is the exact dot product of the decoded weights with activations rounded to 16 bits relative to the
-// largest magnitude of their superblock, as in gemv_i8.cu.
+// The result is the exact dot product of the decoded weights with activations rounded to 16 (IQ4: 31) bits relative to
+// the largest magnitude of their superblock, as in gemv_i8.cu.
 //
 // Organisation: the activations are prepared once per projection by k_prep_nt (16-bit integers in the order the
 // B fragments are read; optionally the row's rmsnorm, the gated unit of two inputs, or only the rows of the
@@ -58,8 +58,8 @@ template <> struct StageNT<FQ_Q6_K> { // per row ql[128] | qh[64] | scales[16]; 
     static constexpr uint32_t ROW = 208, BYTES = WeightRing<FQ_Q6_K, 208>::BYTES;
 };
 
-// Activation rows a block of `nt` tiles serves (0: packed).
-__host__ __device__ constexpr uint32_t nt_rows(int fmt, int nt) { return nt ? 8u * nt : fmt == FQ_IQ4_XS || fmt == FQ_IQ4_NL ? 2u : 4u; }
+// Activation rows a block of `nt` tiles serves (0 and -1: packed into one or two MMA tiles).
+__host__ __device__ constexpr uint32_t nt_rows(int fmt, int nt) { return nt > 0 ? 8u * nt : nt < 0 ? 4u : fmt == FQ_IQ4_XS || fmt == FQ_IQ4_NL ? 2u : 4u; }
 template <int FMT> constexpr bool is_iq4 = FMT == FQ_IQ4_XS || FMT == FQ_IQ4_NL;
 template <> struct StageNT<FQ_IQ4_XS> { // per row nibbles[128] | scales[8]: 144 bytes put the 4-byte reads of eight rows on different banks
     static constexpr uint32_t ROW = 144, BYTES = WeightRing<FQ_IQ4_XS, 144>::BYTES;
@@ -115,14 +115,14 @@ __device__ __forceinline__ void mma_s8s8_k16_z(int (&c)[4], uint32_t a0, uint32_
 //                                                      Q4_K  values 8t .. 8t+7:               hi[8] | lo[8]
 //                                                      Q6_K  values 4t .. 4t+3 of each half:  hi[4] | hi[4] | lo[4] | lo[4]
 //                                                      IQ4   values 4t, 4t+16, 4t+1, 4t+17, .. 4t+19 (the order in which a
-//                                                            pair of nibble bytes decodes):   hi[8] | mid[8]
-//   low  [nblk][8 groups of 32][4 threads][8 bytes]    IQ4 only: the third byte plane, lo[8]
+//                                                            pair of nibble bytes decodes):   p0[8] | p1[8]
+//   low  [nblk][8 groups of 32][4 threads][16 bytes]   IQ4 only: the lower two planes, p2[8] | p3[8]
 //   rec  [nblk][32 bytes]   per superblock: the sums of x' per 32 values as three signed base-256 digits, most
 //                           significant first, 8 bytes each (the B operand of the MMA that multiplies them with
 //                           the eight Q4_K minimums), then 1 / s as f32, then 4 spare bytes.
 // A block copies the superblocks of its slice of TOK = 8 NT rows into shared memory: frag rows with stride
 // 512 nb + 64 (rows g, g + 1 of a quarter-warp on different banks), rec rows with a stride of 4 words mod 32.
-// The IQ4 formats carry activations as 24-bit integers (three planes): their verify widths ran on fp32 products before.
+// The IQ4 formats carry activations as 31-bit integers (four planes): their other kernels multiply in fp32.
 struct PrepNT {
     uint32_t cols, nblk, low_off, rec_off, token_bytes;
 };
@@ -131,7 +131,7 @@ __host__ __device__ inline PrepNT prep_nt_layout(uint32_t cols, bool wide) {
     L.cols = cols;
     L.nblk = cols / 256;
     L.low_off = L.nblk * 512;
-    L.rec_off = L.low_off + (wide ? L.nblk * 256 : 0);
+    L.rec_off = L.low_off + (wide ? L.nblk * 512 : 0);
     L.token_bytes = L.rec_off + L.nblk * 32;
     return L;
 }
@@ -139,16 +139,14 @@ struct ActSmem {
     uint8_t *frag;
     uint8_t *low; // IQ4 only
     uint8_t *rec;
-    uint32_t row_stride, low_stride, rec_stride;
+    uint32_t row_stride, rec_stride;
 };
 // 16 bytes past a multiple of 128: rows stay 16-byte aligned for the copies, and the eight rows a warp reads
 // records of fall on different banks.
 __host__ __device__ inline uint32_t nt_rec_stride(uint32_t nb) { return 32 * nb + ((16 + 128 - (32 * nb) % 128) % 128); } // bytes
-// Bytes of the resident set (a multiple of 16: the warps' rings follow it).  `low` rows: 32 bytes past a multiple of
-// 256, so that the 8-byte reads of four rows fall on different banks.
-__host__ __device__ inline uint32_t nt_low_stride(uint32_t nb, bool wide) { return wide ? nb * 256 + 32 : 0; }
+// Bytes of the resident set (a multiple of 16: the warps' rings follow it); `low` rows lie as `frag` rows do.
 __host__ __device__ inline uint32_t nt_act_bytes(uint32_t tok, uint32_t nb, bool wide) {
-    return (tok * (nb * 512 + 64) + tok * nt_low_stride(nb, wide) + tok * nt_rec_stride(nb) + 15u) & ~15u;
+    return (tok * (nb * 512 + 64) * (wide ? 2 : 1) + tok * nt_rec_stride(nb) + 15u) & ~15u;
 }
 
 // One superblock of one activation row by one warp: lane l holds the eight values at 8 l, already loaded.
@@ -179,17 +177,17 @@ __device__ __forceinline__ void prep_nt_superblock(const float4 &v0, const float
         // the two lays down thread 2 (l % 4)'s run, the second the run of the thread after it.
         const Quant8Wide q = quantize8_wide(v);
         const bool second = lane & 2;
-        auto run = [&](const uint8_t *p) {
-            const uint32_t keep = pack4(second ? p + 4 : p), got = __shfl_xor_sync(0xffffffffu, pack4(second ? p : p + 4), 2);
+        auto run = [&](const uint32_t (&p)[2]) {
+            const uint32_t keep = second ? p[1] : p[0], got = __shfl_xor_sync(0xffffffffu, second ? p[0] : p[1], 2);
             const uint32_t l16 = second ? got : keep, h16 = second ? keep : got; // values below and from 16 on
             return make_uint2(__byte_perm(l16, h16, 0x5140), __byte_perm(l16, h16, 0x7362));
         };
-        const uint2 hi = run(q.hi), mid = run(q.mid), lo = run(q.lo);
+        const uint2 p0 = run(q.p[0]), p1 = run(q.p[1]), p2 = run(q.p[2]), p3 = run(q.p[3]);
         const uint32_t at = 4 * (lane >> 2) + 2 * (lane & 1) + (second ? 1 : 0);
-        *reinterpret_cast<uint4 *>(frag + 16 * at) = make_uint4(hi.x, hi.y, mid.x, mid.y);
-        *reinterpret_cast<uint2 *>(low + 8 * at) = lo;
+        *reinterpret_cast<uint4 *>(frag + 16 * at) = make_uint4(p0.x, p0.y, p1.x, p1.y);
+        *reinterpret_cast<uint4 *>(low + 16 * at) = make_uint4(p2.x, p2.y, p3.x, p3.y);
         if (lane == 0) {
-            *reinterpret_cast<float *>(rec + 24) = q.finite ? ldexpf(1.f, -q.e) : __int_as_float(0x7fc00000);
+            *reinterpret_cast<float *>(rec + 24) = q.inv;
             *reinterpret_cast<uint32_t *>(rec + 28) = 0u;
         }
     } else {
@@ -245,7 +243,7 @@ k_prep_nt(const float *__restrict__ x, const float *__restrict__ x_up, const flo
     const float4 *sp = reinterpret_cast<const float4 *>(x + at + lane * 8);
     uint8_t *base = out + (size_t)xr * L.token_bytes;
     prep_nt_superblock<FMT>(sp[0], sp[1], x_up ? x_up + at : nullptr, norm_w ? norm_w + (size_t)b * 256 : nullptr, scale, lane, base + (size_t)b * 512,
-                            base + L.low_off + (size_t)b * 256, base + L.rec_off + (size_t)b * 32);
+                            base + L.low_off + (size_t)b * 512, base + L.rec_off + (size_t)b * 32);
 }
 
 // The IQ4_XS sub-block scales of a row's header (d | scales_h in h.x, scales_l in h.y) as signed bytes: .x holds
@@ -257,9 +255,33 @@ __device__ __forceinline__ uint2 iq4xs_scales(const uint2 &h) {
     auto minus32 = [](uint32_t v) { return ((v | 0x80808080u) - 0x20202020u) ^ 0x80808080u; }; // byte by byte
     return make_uint2(minus32(even), minus32(odd));
 }
-// IQ4_NL: integers below 2^22 become floats by starting their accumulator at the bits of 1.5 * 2^23 (and
+// The IQ4 formats: integers below 2^22 become floats by starting their accumulator at the bits of 1.5 * 2^23 (and
 // subtracting that), which keeps the conversion unit out of the loop.
 constexpr int IQ4_MAGIC = 0x4B400000;
+// 2^24 c0 + 2^16 c1 + 2^8 c2 + c3 of four such accumulators.  The lower two are added with their offsets still in (257
+// times 1.5 * 2^23 is an fp32 number); the sum is then rounded to a multiple of 256: half of that, against
+// products of 2^31 with a codebook value, once per 32 activations.
+__device__ __forceinline__ float iq4_planes(int c0, int c1, int c2, int c3) {
+    constexpr float BIAS = 12582912.f;
+    const float low = fmaf(256.f, __int_as_float(c2), __int_as_float(c3)) - 257.f * BIAS;
+    return fmaf(16777216.f, __int_as_float(c0) - BIAS, fmaf(65536.f, __int_as_float(c1) - BIAS, low));
+}
+
+// What a superblock with infinite activations and no NaN contributes: the fp32 products of its infinities with the weights
+// of the stage row `row` added up, which the finite values do not change.  `sign`: its p0 plane (Quant8Wide).
+template <int FMT> __device__ __noinline__ float iq4_infinite(const uint8_t *row, const uint8_t *sign) {
+    float sum = 0.f;
+    for (int i = 0; i < 256; i++) { // byte i of the plane: group i / 32, thread (i / 8) % 4, its value i % 8
+        const int j = i >> 5, t = (i >> 3) & 3, s = (int)(int8_t)sign[64 * j + 16 * t + (i & 7)];
+        if (s == 0) continue;
+        const int pair = 4 * t + ((i & 7) >> 1); // the nibble byte; odd values are its high half
+        const uint32_t nibble = (i & 1) ? row[16 * j + pair] >> 4 : row[16 * j + pair] & 15u;
+        const uint8_t *hdr = row + 128;
+        const float d = FMT == FQ_IQ4_XS ? load_f16(hdr) * (float)iq4xs_scale(hdr, j) : load_f16(hdr + 2 * j);
+        sum += d * iq4_value(nibble) * (s > 0 ? INFINITY : -INFINITY);
+    }
+    return sum;
+}
 
 // One superblock (index `bb` within the block's slice) of a 16-row tile whose packed bytes lie in `stage`,
 // against NT tiles of eight activation rows: adds into yacc[nt][i], i = 2 r + c, the contribution to weight row
@@ -355,12 +377,9 @@ __device__ __forceinline__ void superblock_nt(const uint8_t *stage, const ActSme
     } else if constexpr (is_iq4<FMT>) {
         constexpr uint32_t ROW = StageNT<FMT>::ROW;
         const uint8_t *r0 = stage + g * ROW, *r1 = r0 + 8 * ROW;
-        const uint8_t *lowp[NT];
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++) lowp[nt] = A.low + (size_t)(8 * nt + g) * A.low_stride + (size_t)bb * 256 + 8 * t;
-        // IQ4_XS: the sub-blocks' signed scales and d.  IQ4_NL: a sub-block is a block with an f16 d of its own.
+        // A row's factor and its sub-blocks': d and the signed scales of IQ4_XS, 1 and the blocks' own d of IQ4_NL.
         uint2 sc4[2];
-        float d[2] = {0.f, 0.f};
+        float d[2] = {1.f, 1.f};
         uint4 dn[2];
 #pragma unroll
         for (int r = 0; r < 2; r++) {
@@ -373,44 +392,46 @@ __device__ __forceinline__ void superblock_nt(const uint8_t *stage, const ActSme
                 dn[r] = *reinterpret_cast<const uint4 *>(hp);
             }
         }
-        int am[NT][4];
+        // IQ4_XS adds up scale * plane in integers, IQ4_NL its planes' sum times d in floats.
+        constexpr bool INT = FMT == FQ_IQ4_XS && NT <= 2;
+        constexpr int INIT = INT ? 0 : IQ4_MAGIC;
         float fa[NT][4];
+        int ia[INT ? NT : 1][4][4];
 #pragma unroll
         for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-            for (int i = 0; i < 4; i++) am[nt][i] = 0, fa[nt][i] = 0.f;
+            for (int i = 0; i < 4; i++) {
+                fa[nt][i] = 0.f;
+                if constexpr (INT)
+                    for (int p = 0; p < 4; p++) ia[nt][p][i] = 0;
+            }
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const uint2 v0 = iq4_lookup8(*reinterpret_cast<const uint32_t *>(r0 + 16 * j + 4 * t));
             const uint2 v1 = iq4_lookup8(*reinterpret_cast<const uint32_t *>(r1 + 16 * j + 4 * t));
-            constexpr int INIT = FMT == FQ_IQ4_NL ? IQ4_MAGIC : 0;
-            int s0 = 0, s1 = 0;
-            float d0 = 0.f, d1 = 0.f;
-            if constexpr (FMT == FQ_IQ4_XS) {
-                s0 = byte_s((j & 1) ? sc4[0].y : sc4[0].x, j >> 1);
-                s1 = byte_s((j & 1) ? sc4[1].y : sc4[1].x, j >> 1);
-            } else {
-                d0 = f16_bits_to_f32((uint16_t)(word_of(dn[0], j >> 1) >> (16 * (j & 1))));
-                d1 = f16_bits_to_f32((uint16_t)(word_of(dn[1], j >> 1) >> (16 * (j & 1))));
+            float s[2] = {0.f, 0.f};
+            int si[2] = {0, 0};
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                if constexpr (INT) si[r] = byte_s((j & 1) ? sc4[r].y : sc4[r].x, j >> 1);
+                else s[r] = f16_bits_to_f32((uint16_t)(word_of(dn[r], j >> 1) >> (16 * (j & 1))));
             }
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const uint4 f = *reinterpret_cast<const uint4 *>(fragp[nt] + 64 * j);
-                const uint2 fl = *reinterpret_cast<const uint2 *>(lowp[nt] + 32 * j);
-                int ch[4], cm[4], cl[4];
-                mma_s8s8_i(ch, v0.x, v1.x, v0.y, v1.y, f.x, f.y, INIT);
-                mma_s8s8_i(cm, v0.x, v1.x, v0.y, v1.y, f.z, f.w, INIT);
-                mma_s8s8_i(cl, v0.x, v1.x, v0.y, v1.y, fl.x, fl.y, INIT);
+                const uint4 fh = *reinterpret_cast<const uint4 *>(fragp[nt] + 64 * j);
+                const uint4 fl = *reinterpret_cast<const uint4 *>(fragp[nt] + (A.low - A.frag) + 64 * j);
+                int c[4][4];
+                mma_s8s8_i(c[0], v0.x, v1.x, v0.y, v1.y, fh.x, fh.y, INIT);
+                mma_s8s8_i(c[1], v0.x, v1.x, v0.y, v1.y, fh.z, fh.w, INIT);
+                mma_s8s8_i(c[2], v0.x, v1.x, v0.y, v1.y, fl.x, fl.y, INIT);
+                mma_s8s8_i(c[3], v0.x, v1.x, v0.y, v1.y, fl.z, fl.w, INIT);
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    if constexpr (FMT == FQ_IQ4_XS) {
-                        ah[nt][i] += (i < 2 ? s0 : s1) * ch[i];
-                        am[nt][i] += (i < 2 ? s0 : s1) * cm[i];
-                        al[nt][i] += (i < 2 ? s0 : s1) * cl[i];
+                    if constexpr (INT) {
+#pragma unroll
+                        for (int p = 0; p < 4; p++) ia[nt][p][i] += si[i >> 1] * c[p][i];
                     } else {
-                        const float bias = __int_as_float(IQ4_MAGIC);
-                        const float dot = fmaf(65536.f, __int_as_float(ch[i]) - bias, fmaf(256.f, __int_as_float(cm[i]) - bias, __int_as_float(cl[i]) - bias));
-                        fa[nt][i] = fmaf(i < 2 ? d0 : d1, dot, fa[nt][i]);
+                        fa[nt][i] = fmaf(s[i >> 1], iq4_planes(c[0][i], c[1][i], c[2][i], c[3][i]), fa[nt][i]);
                     }
                 }
             }
@@ -419,10 +440,13 @@ __device__ __forceinline__ void superblock_nt(const uint8_t *stage, const ActSme
         for (int nt = 0; nt < NT; nt++)
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const float inv = *reinterpret_cast<const float *>(A.rec + (size_t)(8 * nt + 2 * t + (i & 1)) * A.rec_stride + (size_t)bb * 32 + 24);
-                if constexpr (FMT == FQ_IQ4_XS)
-                    yacc[nt][i] = fmaf(inv * d[i >> 1], fmaf(65536.f, (float)ah[nt][i], fmaf(256.f, (float)am[nt][i], (float)al[nt][i])), yacc[nt][i]);
-                else yacc[nt][i] = fmaf(inv, fa[nt][i], yacc[nt][i]);
+                const uint32_t tok = 8 * nt + 2 * t + (i & 1);
+                const float inv = *reinterpret_cast<const float *>(A.rec + (size_t)tok * A.rec_stride + (size_t)bb * 32 + 24);
+                if constexpr (INT)
+                    fa[nt][i] = fmaf(16777216.f, (float)ia[nt][0][i], fmaf(65536.f, (float)ia[nt][1][i], fmaf(256.f, (float)ia[nt][2][i], (float)ia[nt][3][i])));
+                // inv last: alone it may be as small as 2^-149, and the product with d would lose bits.
+                if (inv < INFINITY) yacc[nt][i] = fmaf(inv, d[i >> 1] * fa[nt][i], yacc[nt][i]);
+                else yacc[nt][i] += inv != inv ? inv : iq4_infinite<FMT>(i < 2 ? r0 : r1, A.frag + (size_t)tok * A.row_stride + (size_t)bb * 512);
             }
     } else {
         const uint8_t *r0 = stage + g * 208, *r1 = r0 + 8 * 208;
@@ -489,27 +513,16 @@ __device__ __forceinline__ void superblock_nt(const uint8_t *stage, const ActSme
 
 // The same superblock against at most eight (row, plane) pairs of activations: the planes of a row sit in different
 // COLUMNS of one MMA instead of in MMAs of their own, so that a scale group costs one MMA and four multiply-adds, not
-// two or three of each (17408 x 5120 Q4_K, two rows: 19.0 -> 15.7 us; four rows 19.6 -> 17.6 us).  Column c is plane c % P of row c / P, with P = 2 (up to four rows), or for the IQ4 formats
-// P = 4 of which the last is zero (up to two rows).  Thread t so gets both planes of row t, or planes 2 (t % 2) and
-// 2 (t % 2) + 1 of row t / 2 (the caller adds the two threads' sums): adds into yacc[r] the contribution to weight
-// row g + 8 r.  Five rows and more take superblock_nt.
+// two or four of each (17408 x 5120 Q4_K, two rows: 19.0 -> 15.7 us; four rows 19.6 -> 17.6 us).  Column c is plane c % 2
+// of row c / 2 (up to four rows): thread t gets both planes of row t.  IQ4: superblock_pack_iq4.  Adds into yacc[r] the
+// contribution to weight row g + 8 r.  More rows take superblock_nt.
 template <int FMT>
 __device__ __forceinline__ void superblock_pack(const uint8_t *stage, const ActSmem &A, uint32_t bb, bool odd_b, int g, int t, float (&yacc)[2]) {
-    constexpr bool WIDE = is_iq4<FMT>;
-    const uint32_t col_row = WIDE ? (uint32_t)g >> 2 : (uint32_t)g >> 1, plane = WIDE ? g & 3 : g & 1, my_row = WIDE ? (uint32_t)t >> 1 : (uint32_t)t;
-    // What this thread feeds of a 32-value group j: eight bytes at fp + fstep * j.
-    const uint8_t *fp = A.frag + (size_t)col_row * A.row_stride + (size_t)bb * 512 + 16 * t + 8 * (plane & 1);
-    uint32_t fstep = 64;
-    if (WIDE && plane >= 2) {
-        fp = A.low + (size_t)col_row * A.low_stride + (size_t)bb * 256 + 8 * t;
-        fstep = 32;
-    }
-    auto feed = [&](int j) {
-        uint2 f = *reinterpret_cast<const uint2 *>(fp + fstep * j);
-        if (WIDE && plane == 3) f = make_uint2(0u, 0u);
-        return f;
-    };
-    const float inv = *reinterpret_cast<const float *>(A.rec + (size_t)my_row * A.rec_stride + (size_t)bb * 32 + 24);
+    const uint32_t col_row = (uint32_t)g >> 1;
+    // What this thread feeds of a 32-value group j: eight bytes.
+    const uint8_t *fp = A.frag + (size_t)col_row * A.row_stride + (size_t)bb * 512 + 16 * t + 8 * (g & 1);
+    auto feed = [&](int j) { return *reinterpret_cast<const uint2 *>(fp + 64 * j); };
+    const float inv = *reinterpret_cast<const float *>(A.rec + (size_t)t * A.rec_stride + (size_t)bb * 32 + 24);
     int acc[4] = {0, 0, 0, 0};
     if constexpr (FMT == FQ_Q4_K || FMT == FQ_Q5_K) {
         constexpr uint32_t ROW = StageNT<FMT>::ROW, QS = FMT == FQ_Q4_K ? 16 : 48;
@@ -571,48 +584,6 @@ __device__ __forceinline__ void superblock_pack(const uint8_t *stage, const ActS
             const float dot = fmaf(256.f, (float)acc[2 * r], (float)acc[2 * r + 1]);
             yacc[r] = fmaf(inv, d[r] * dot - dmin[r] * (float)mins, yacc[r]);
         }
-    } else if constexpr (WIDE) {
-        constexpr uint32_t ROW = StageNT<FMT>::ROW;
-        const uint8_t *r0 = stage + g * ROW, *r1 = r0 + 8 * ROW;
-        uint2 sc4[2];
-        float d[2] = {0.f, 0.f}, facc[2] = {0.f, 0.f};
-        uint4 dn[2];
-        const float w0 = (t & 1) ? 1.f : 65536.f, w1 = (t & 1) ? 0.f : 256.f; // of this thread's two planes
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            const uint8_t *hp = (r ? r1 : r0) + 128;
-            if constexpr (FMT == FQ_IQ4_XS) {
-                const uint2 h = *reinterpret_cast<const uint2 *>(hp);
-                d[r] = f16_bits_to_f32((uint16_t)(h.x & 0xFFFFu));
-                sc4[r] = iq4xs_scales(h);
-            } else {
-                dn[r] = *reinterpret_cast<const uint4 *>(hp);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint2 v0 = iq4_lookup8(*reinterpret_cast<const uint32_t *>(r0 + 16 * j + 4 * t));
-            const uint2 v1 = iq4_lookup8(*reinterpret_cast<const uint32_t *>(r1 + 16 * j + 4 * t));
-            const uint2 f = feed(j);
-            int ci[4];
-            mma_s8s8_i(ci, v0.x, v1.x, v0.y, v1.y, f.x, f.y, FMT == FQ_IQ4_NL ? IQ4_MAGIC : 0);
-#pragma unroll
-            for (int r = 0; r < 2; r++) {
-                if constexpr (FMT == FQ_IQ4_XS) {
-                    const int sc = byte_s((j & 1) ? sc4[r].y : sc4[r].x, j >> 1);
-                    acc[2 * r] += sc * ci[2 * r];
-                    acc[2 * r + 1] += sc * ci[2 * r + 1];
-                } else {
-                    const float bias = __int_as_float(IQ4_MAGIC), dj = f16_bits_to_f32((uint16_t)(word_of(dn[r], j >> 1) >> (16 * (j & 1))));
-                    facc[r] = fmaf(dj, fmaf(w0, __int_as_float(ci[2 * r]) - bias, w1 * (__int_as_float(ci[2 * r + 1]) - bias)), facc[r]);
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            if constexpr (FMT == FQ_IQ4_XS) yacc[r] = fmaf(inv * d[r], fmaf(w0, (float)acc[2 * r], w1 * (float)acc[2 * r + 1]), yacc[r]);
-            else yacc[r] = fmaf(inv, facc[r], yacc[r]);
-        }
     } else {
         const uint8_t *r0 = stage + g * 208, *r1 = r0 + 8 * 208;
         float d4[2];
@@ -659,8 +630,68 @@ __device__ __forceinline__ void superblock_pack(const uint8_t *stage, const ActS
     }
 }
 
+// IQ4 formats: `PT` MMA tiles of two rows each, column c of tile q is plane c % 4 of row 2 q + c / 4.  Thread t gets planes
+// 2 (t % 2) and 2 (t % 2) + 1 of row 2 q + t / 2 (the caller adds the two threads' sums): adds into yacc[2 q + r] the
+// contribution to weight row g + 8 r.
+template <int FMT, int PT>
+__device__ __forceinline__ void superblock_pack_iq4(const uint8_t *stage, const ActSmem &A, uint32_t bb, int g, int t, float (&yacc)[2 * PT]) {
+    constexpr uint32_t ROW = StageNT<FMT>::ROW;
+    const uint8_t *r0 = stage + g * ROW, *r1 = r0 + 8 * ROW;
+    const uint8_t *fp = ((g & 2) ? A.low : A.frag) + (size_t)((uint32_t)g >> 2) * A.row_stride + (size_t)bb * 512 + 16 * t + 8 * (g & 1);
+    uint2 sc4[2];
+    float d[2] = {1.f, 1.f}, facc[PT][2] = {};
+    int acc[PT][4] = {};
+    uint4 dn[2];
+    const float w0 = (t & 1) ? 256.f : 16777216.f, w1 = (t & 1) ? 1.f : 65536.f; // of this thread's two planes
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+        const uint8_t *hp = (r ? r1 : r0) + 128;
+        if constexpr (FMT == FQ_IQ4_XS) {
+            const uint2 h = *reinterpret_cast<const uint2 *>(hp);
+            d[r] = f16_bits_to_f32((uint16_t)(h.x & 0xFFFFu));
+            sc4[r] = iq4xs_scales(h);
+        } else {
+            dn[r] = *reinterpret_cast<const uint4 *>(hp);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const uint2 v0 = iq4_lookup8(*reinterpret_cast<const uint32_t *>(r0 + 16 * j + 4 * t));
+        const uint2 v1 = iq4_lookup8(*reinterpret_cast<const uint32_t *>(r1 + 16 * j + 4 * t));
+#pragma unroll
+        for (int q = 0; q < PT; q++) {
+            const uint2 f = *reinterpret_cast<const uint2 *>(fp + (size_t)(2 * q) * A.row_stride + 64 * j);
+            int ci[4];
+            mma_s8s8_i(ci, v0.x, v1.x, v0.y, v1.y, f.x, f.y, FMT == FQ_IQ4_NL ? IQ4_MAGIC : 0);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                if constexpr (FMT == FQ_IQ4_XS) {
+                    const int sc = byte_s((j & 1) ? sc4[r].y : sc4[r].x, j >> 1);
+                    acc[q][2 * r] += sc * ci[2 * r];
+                    acc[q][2 * r + 1] += sc * ci[2 * r + 1];
+                } else {
+                    const float bias = __int_as_float(IQ4_MAGIC), dj = f16_bits_to_f32((uint16_t)(word_of(dn[r], j >> 1) >> (16 * (j & 1))));
+                    facc[q][r] = fmaf(dj, fmaf(w0, __int_as_float(ci[2 * r]) - bias, w1 * (__int_as_float(ci[2 * r + 1]) - bias)), facc[q][r]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < PT; q++) {
+        const uint32_t my_row = 2 * q + ((uint32_t)t >> 1);
+        const float inv = *reinterpret_cast<const float *>(A.rec + (size_t)my_row * A.rec_stride + (size_t)bb * 32 + 24);
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const float dot = FMT == FQ_IQ4_XS ? fmaf(w0, (float)acc[q][2 * r], w1 * (float)acc[q][2 * r + 1]) : facc[q][r];
+            if (inv < INFINITY) yacc[2 * q + r] = fmaf(inv, d[r] * dot, yacc[2 * q + r]);
+            else if (!(t & 1)) // once per row
+                yacc[2 * q + r] += inv != inv ? inv : iq4_infinite<FMT>(r ? r1 : r0, A.frag + (size_t)my_row * A.row_stride + (size_t)bb * 512);
+        }
+    }
+}
+
 // FMT: a format of nt_format(); NT: tiles of eight activation rows, or 0: up to four (IQ4: two) rows packed into one
-// tile (superblock_pack); STAGES: superblocks in flight per warp;
+// tile, or -1 (IQ4): up to four rows packed into two; STAGES: superblocks in flight per warp;
 // GROUPED: block = (expert, tile of 8 NT expert-sorted rows), else block = (K slice, share of the row tiles).
 template <int FMT, int NT, int STAGES, bool GROUPED>
 __global__ void __launch_bounds__(NT > 2 ? 384 : 512, 1)
@@ -731,11 +762,10 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
 
     ActSmem A;
     A.row_stride = J.nb_max * 512 + 64;
-    A.low_stride = nt_low_stride(J.nb_max, WIDE);
     A.rec_stride = nt_rec_stride(J.nb_max);
     A.frag = nt_smem;
     A.low = A.frag + (size_t)TOK * A.row_stride;
-    A.rec = A.low + (size_t)TOK * A.low_stride;
+    A.rec = A.low + (WIDE ? (size_t)TOK * A.row_stride : 0);
     uint8_t *ring = nt_smem + nt_act_bytes(TOK, J.nb_max, WIDE) + (size_t)warp * STAGES * St::BYTES;
 
     struct Tile {
@@ -783,9 +813,9 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
     if constexpr (!GROUPED) pdl_wait();
     const uint32_t seq = P.world > 1 ? tp_seq(P) : 0u;
 
-    // The block's resident activations: 16-byte pieces of the prepared rows (per row 32 nb of fragments, 16 nb of the
-    // third plane where there is one, 2 nb of records), copied asynchronously; rows the job does not have are zero.
-    if (NT == 0 && J.x) {
+    // The block's resident activations: 16-byte pieces of the prepared rows (per row 32 nb of fragments, as many of
+    // the lower planes where there are such, 2 nb of records), copied asynchronously; rows the job does not have are zero.
+    if (NT <= 0 && J.x) {
         // Few rows: preparing the slice here (a warp per row and superblock) is cheaper than a launch that does it.
         __shared__ float norm_part[NORM_WARPS];
         float scale0 = 0.f, scale1 = 0.f; // with a norm there are at most two rows
@@ -802,12 +832,16 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
             const float4 *sp = reinterpret_cast<const float4 *>(J.x + at + lane * 8);
             prep_nt_superblock<FMT>(sp[0], sp[1], J.x_up ? J.x_up + at : nullptr, J.norm_w ? J.norm_w + (size_t)(b0 + b) * 256 : nullptr,
                                     tok ? scale1 : scale0, lane, A.frag + (size_t)tok * A.row_stride + (size_t)b * 512,
-                                    A.low + (size_t)tok * A.low_stride + (size_t)b * 256, A.rec + (size_t)tok * A.rec_stride + (size_t)b * 32);
+                                    A.low + (size_t)tok * A.row_stride + (size_t)b * 512, A.rec + (size_t)tok * A.rec_stride + (size_t)b * 32);
         }
+        // Rows the job does not have: whatever lies there counts nothing (and no infinity).
+        if constexpr (WIDE)
+            for (uint32_t i = threadIdx.x; i < (TOK - m) * nb; i += blockDim.x)
+                *reinterpret_cast<float *>(A.rec + (size_t)(m + i / nb) * A.rec_stride + (size_t)(i % nb) * 32 + 24) = 0.f;
     } else {
-        // Rows the tile loop will read: all of them, or (grouped tiles of 32) as many eights as it will take.
-        const uint32_t rows_used = (GROUPED && NT == 4) ? (m <= 8 ? 8u : m <= 16 ? 16u : 32u) : TOK;
-        const uint32_t frags = 32 * nb, lows = WIDE ? 16 * nb : 0, per_row = frags + lows + 2 * nb, pieces = rows_used * per_row;
+        // Rows the tile loop will read: all of them, or (grouped tiles) as many eights as it will take.
+        const uint32_t rows_used = GROUPED ? (m <= 8 ? 8u : m <= 16 ? 16u : 32u) : TOK;
+        const uint32_t frags = 32 * nb, lows = WIDE ? 32 * nb : 0, per_row = frags + lows + 2 * nb, pieces = rows_used * per_row;
         const PrepNT L = prep_nt_layout(J.cols, WIDE);
         for (uint32_t i = threadIdx.x; i < pieces; i += blockDim.x) {
             const uint32_t tok = i / per_row, p = i - tok * per_row;
@@ -817,8 +851,8 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
                 dst = A.frag + (size_t)tok * A.row_stride + 16 * p;
                 from = (size_t)b0 * 512 + 16 * p;
             } else if (p < frags + lows) {
-                dst = A.low + (size_t)tok * A.low_stride + 16 * (p - frags);
-                from = L.low_off + (size_t)b0 * 256 + 16 * (p - frags);
+                dst = A.low + (size_t)tok * A.row_stride + 16 * (p - frags);
+                from = L.low_off + (size_t)b0 * 512 + 16 * (p - frags);
             } else {
                 dst = A.rec + (size_t)tok * A.rec_stride + 16 * (p - frags - lows);
                 from = L.rec_off + (size_t)b0 * 32 + 16 * (p - frags - lows);
@@ -836,16 +870,16 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
     }
     __syncthreads();
 
-    // The tile loop for NTU tiles of eight activation rows (0: packed).  A grouped block picks NTU by the rows its tile
+    // The tile loop for NTU tiles of eight activation rows (0, -1: packed).  A grouped block picks NTU by the rows its tile
     // holds (the resident layout does not depend on it), so a nearly empty tile does not pay for a full one.
     uint32_t c_stage = 0;
     auto run = [&](auto ntu) {
-        constexpr int NTU = decltype(ntu)::value, NV = NTU ? 4 * NTU : 2; // a lane's values
+        constexpr int NTU = decltype(ntu)::value, PT = NTU < 0 ? 2 : 1, NV = NTU > 0 ? 4 * NTU : 2 * PT; // a lane's values
         for (uint32_t tile = first; tile < total_tiles; tile += stride) {
             const Tile here = tile_at(tile);
             float v[NV];
             {
-                float yacc[NTU ? NTU : 1][4], ypack[2] = {0.f, 0.f};
+                float yacc[NTU > 0 ? NTU : 1][4], ypack[2 * PT] = {};
 #pragma unroll
                 for (int nt = 0; nt < NTU; nt++)
 #pragma unroll
@@ -856,14 +890,15 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
                     __syncwarp();
                     const uint8_t *stage = ring + (size_t)c_stage * St::BYTES;
                     const bool odd_b = ((b0 + bb) & 1u) != 0;
-                    if constexpr (NTU == 0) superblock_pack<FMT>(stage, A, bb, odd_b, g, t, ypack);
+                    if constexpr (NTU <= 0 && WIDE) superblock_pack_iq4<FMT, PT>(stage, A, bb, g, t, ypack);
+                    else if constexpr (NTU <= 0) superblock_pack<FMT>(stage, A, bb, odd_b, g, t, ypack);
                     else superblock_nt<FMT, NTU>(stage, A, bb, odd_b, g, t, yacc);
                     __syncwarp();
                     c_stage = c_stage + 1 == STAGES ? 0 : c_stage + 1;
                 }
 #pragma unroll
-                for (int i = 0; i < NV; i++) v[i] = NTU ? yacc[NTU ? i / 4 : 0][i % 4] : ypack[i & 1];
-                if constexpr (NTU == 0 && WIDE) // two threads hold a row's planes
+                for (int i = 0; i < NV; i++) v[i] = NTU > 0 ? yacc[NTU > 0 ? i / 4 : 0][i % 4] : ypack[NTU > 0 ? 0 : i];
+                if constexpr (NTU <= 0 && WIDE) // two threads hold a row's planes
                     for (int i = 0; i < NV; i++) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 1);
             }
             bool store = true;
@@ -895,8 +930,8 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
             if (store) {
 #pragma unroll
                 for (int i = 0; i < NV; i++) {
-                    const uint32_t row = here.row0 + g + (NTU ? (i % 4) >> 1 : i) * 8;
-                    const uint32_t tok = NTU ? 8 * (i / 4) + 2 * t + (i & 1) : WIDE ? (t & 1 ? TOK : t >> 1) : t;
+                    const uint32_t row = here.row0 + g + (NTU > 0 ? (i % 4) >> 1 : i & 1) * 8;
+                    const uint32_t tok = NTU > 0 ? 8 * (i / 4) + 2 * t + (i & 1) : WIDE ? (t & 1 ? TOK : 2 * (i >> 1) + (t >> 1)) : t;
                     if (row < here.rows && tok < m) {
                         float *dst = &here.y[(size_t)(xrow0 + tok) * here.rows + row];
                         *dst = v[i];
@@ -906,10 +941,10 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
             }
         }
     };
-    if constexpr (GROUPED && NT == 4) {
+    if constexpr (GROUPED) {
         if (m <= 8) run(std::integral_constant<int, 1>{});
-        else if (m <= 16) run(std::integral_constant<int, 2>{});
-        else run(std::integral_constant<int, 4>{});
+        else if (NT == 2 || m <= 16) run(std::integral_constant<int, 2>{});
+        else run(std::integral_constant<int, NT>{});
     } else {
         run(std::integral_constant<int, NT>{});
     }
@@ -1013,11 +1048,11 @@ template <int FMT, int NT> int launch_dense(fq_device *dev, const ProjectArgs *a
     J.nb_max = S.nb_max;
     J.ws = (float2 *)dev->nt_ws;
     J.counters = dev->nt_counters;
-    if (S.slices > 1 && ((size_t)tiles * S.slices * 32 * (NT ? 2 * NT : 1) * sizeof(float2) > dev->nt_ws_bytes || tiles > dev->nt_counter_count))
+    if (S.slices > 1 && ((size_t)tiles * S.slices * 32 * (NT > 0 ? 2 * NT : NT < 0 ? 2 : 1) * sizeof(float2) > dev->nt_ws_bytes || tiles > dev->nt_counter_count))
         return FQ_ERR_UNSUPPORTED;
     // Packed widths with one or two superblocks of work per warp: prepared by every block for itself, without a launch
     // (1500 x 2048, two rows: 7.6 -> 5.6 us).
-    const bool own_prep = NT == 0 && a[0].m * S.nb_max <= NT_OWN_PREP * S.warps && (!a[0].norm_w || a[0].m <= 2);
+    const bool own_prep = NT <= 0 && a[0].m * S.nb_max <= NT_OWN_PREP * S.warps && (!a[0].norm_w || a[0].m <= 2);
     if (own_prep) {
         J.x = (const float *)a[0].x;
         J.x_up = a[0].x_up;
@@ -1055,6 +1090,8 @@ int fq_launch_gemv_nt_many(fq_device *dev, const ProjectArgs *a, uint32_t count)
     auto go = [&](auto fmt) {
         constexpr int FMT = decltype(fmt)::value;
         if (f.m <= nt_rows(FMT, 0)) return launch_dense<FMT, 0>(dev, a, count);
+        if constexpr (is_iq4<FMT>)
+            if (f.m <= nt_rows(FMT, -1)) return launch_dense<FMT, -1>(dev, a, count);
         return f.m <= 8 ? launch_dense<FMT, 1>(dev, a, count) : launch_dense<FMT, 2>(dev, a, count);
     };
     switch (f.format) {
@@ -1065,6 +1102,36 @@ int fq_launch_gemv_nt_many(fq_device *dev, const ProjectArgs *a, uint32_t count)
     default: return go(std::integral_constant<int, FQ_IQ4_XS>{});
     }
 }
+
+// Grouped blocks take tiles of 32 expert-sorted rows, or of 16 where 32 of the row's width do not fit beside the rings: the
+// four activation planes of the IQ4 formats from 1536 columns on (Q4_K 2304).
+namespace {
+template <int FMT, int GNT> int launch_grouped(fq_device *dev, NtJob &J, const ProjectArgs &f, uint32_t tiles, const uint32_t *src, uint32_t src_div) {
+    NtShape S;
+    if (!nt_shape<FMT, GNT>(dev, tiles, J.nblk, true, S)) {
+        if constexpr (GNT > 2 && is_iq4<FMT>) return launch_grouped<FMT, 2>(dev, J, f, tiles, src, src_div);
+        return FQ_ERR_UNSUPPORTED;
+    }
+    J.nb_max = S.nb_max;
+    cudaError_t e = cudaSuccess;
+    // With a gather (`src`) every row of x is prepared once and the blocks pick rows by index; else the rows of
+    // the experts in `offsets` (a rank's share when the matrices hold only some experts).
+    if (src) {
+        if (src_div == 0) return FQ_ERR_UNSUPPORTED;
+        J.src = src;
+        J.src_div = src_div;
+        J.prep = launch_prep(dev, FMT, f, (J.total_rows + src_div - 1) / src_div, nullptr, 1, nullptr, 0, e);
+    } else {
+        J.prep = launch_prep(dev, FMT, f, J.total_rows, nullptr, 1, f.offsets, f.groups, e);
+    }
+    if (!J.prep) return FQ_ERR_UNSUPPORTED;
+    if (int rc = fq_check_cuda(dev, e, "activation preparation launch")) return rc;
+    // Every group has at most ceil(rows / tile) <= rows / tile + 1 tiles.
+    const uint32_t grid = J.total_rows / (8 * GNT) + J.groups;
+    if (int rc = fq_check_cuda(dev, nt_launch<FMT, GNT, true>(dev, J, S, grid, TpPush{}), "grouped gemv launch")) return rc;
+    return fq_end_enqueue(dev, "gemv_nt_grouped", 2);
+}
+} // namespace
 
 // Grouped expert projection over expert-sorted rows (F32 in, F32 out), up to two expert stacks of one shape
 // sharing the rows (gate and up).  `src` (may be null): row r of the sorted set is row src[r] / src_div of x, so
@@ -1096,35 +1163,11 @@ int fq_launch_gemv_nt_grouped(fq_device *dev, const ProjectArgs *a, uint32_t cou
     J.slots = f.slots;
     J.groups = f.groups;
     J.total_rows = total_rows;
-    NtShape S;
-    constexpr int GNT = 4; // grouped blocks take tiles of 32 expert-sorted rows
-    const bool ok = f.format == FQ_Q4_K   ? nt_shape<FQ_Q4_K, GNT>(dev, tiles, J.nblk, true, S)
-                  : f.format == FQ_Q5_K   ? nt_shape<FQ_Q5_K, GNT>(dev, tiles, J.nblk, true, S)
-                  : f.format == FQ_Q6_K   ? nt_shape<FQ_Q6_K, GNT>(dev, tiles, J.nblk, true, S)
-                  : f.format == FQ_IQ4_NL ? nt_shape<FQ_IQ4_NL, GNT>(dev, tiles, J.nblk, true, S)
-                                          : nt_shape<FQ_IQ4_XS, GNT>(dev, tiles, J.nblk, true, S);
-    if (!ok) return FQ_ERR_UNSUPPORTED;
-    J.nb_max = S.nb_max;
-    cudaError_t e = cudaSuccess;
-    // With a gather (`src`) every row of x is prepared once and the blocks pick rows by index; else the rows of
-    // the experts in `offsets` (a rank's share when the matrices hold only some experts).
-    if (src) {
-        if (src_div == 0) return FQ_ERR_UNSUPPORTED;
-        J.src = src;
-        J.src_div = src_div;
-        J.prep = launch_prep(dev, (int)f.format, f, (total_rows + src_div - 1) / src_div, nullptr, 1, nullptr, 0, e);
-    } else {
-        J.prep = launch_prep(dev, (int)f.format, f, total_rows, nullptr, 1, f.offsets, f.groups, e);
+    switch (f.format) {
+    case FQ_Q4_K: return launch_grouped<FQ_Q4_K, 4>(dev, J, f, tiles, src, src_div);
+    case FQ_Q5_K: return launch_grouped<FQ_Q5_K, 4>(dev, J, f, tiles, src, src_div);
+    case FQ_Q6_K: return launch_grouped<FQ_Q6_K, 4>(dev, J, f, tiles, src, src_div);
+    case FQ_IQ4_NL: return launch_grouped<FQ_IQ4_NL, 4>(dev, J, f, tiles, src, src_div);
+    default: return launch_grouped<FQ_IQ4_XS, 4>(dev, J, f, tiles, src, src_div);
     }
-    if (!J.prep) return FQ_ERR_UNSUPPORTED;
-    if (int rc = fq_check_cuda(dev, e, "activation preparation launch")) return rc;
-    // Every group has at most ceil(rows / 32) <= rows / 32 + 1 tiles.
-    const uint32_t grid = total_rows / (8 * GNT) + f.groups;
-    e = f.format == FQ_Q4_K   ? nt_launch<FQ_Q4_K, GNT, true>(dev, J, S, grid, TpPush{})
-      : f.format == FQ_Q5_K   ? nt_launch<FQ_Q5_K, GNT, true>(dev, J, S, grid, TpPush{})
-      : f.format == FQ_Q6_K   ? nt_launch<FQ_Q6_K, GNT, true>(dev, J, S, grid, TpPush{})
-      : f.format == FQ_IQ4_NL ? nt_launch<FQ_IQ4_NL, GNT, true>(dev, J, S, grid, TpPush{})
-                              : nt_launch<FQ_IQ4_XS, GNT, true>(dev, J, S, grid, TpPush{});
-    if (int rc = fq_check_cuda(dev, e, "grouped gemv launch")) return rc;
-    return fq_end_enqueue(dev, "gemv_nt_grouped", 2);
 }

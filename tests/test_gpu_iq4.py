@@ -134,6 +134,46 @@ def test_moe_block_with_iq4_xs_experts(device, m):
     assert ref.rel_err(host(out).reshape(m, hidden), want) <= 3 * TOL_F32
 
 
+def _inputs(kind, m, cols, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal((m, cols))
+    if kind == "gated":  # silu(g) * u: long tails
+        g = 1.5 * rng.standard_normal((m, cols))
+        x = g / (1 + np.exp(-g)) * x
+    elif kind == "outliers":
+        x[:, ::97] *= 1000
+    elif kind == "tiny":
+        x *= 1e-30
+    return x.astype(np.float32)
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 16])
+@pytest.mark.parametrize("kind", ["normal", "gated", "outliers", "tiny"])
+@pytest.mark.parametrize("cols", [256, 1024, 2304])
+def test_no_further_from_64_bits_than_fp32(device, fmt, m, kind, cols):
+    """The integer kernels drop less of the activations than the fp32 kernels (`set_exact`) round off, also where one value
+    of a superblock is far above the others and where all are far below one."""
+    s = S()
+    rows = 384
+    packed = ref.random_matrix(fmt, rows, cols, seed=cols)
+    dense = ref.dequant(fmt, packed).reshape(rows, cols).astype(np.float64)
+    w = s.Matrix.from_packed(device, rows, cols, 1, fmt, packed)
+    x = _inputs(kind, m, cols, m)
+    want = x.astype(np.float64) @ dense.T
+    errors = []
+    for exact in (False, True):
+        y = torch.zeros(m, rows, device="cuda")
+        device.set_exact(exact)
+        try:
+            s.project(device, w, dev_f32(x), m, y)
+            device.synchronize()
+        finally:
+            device.set_exact(False)
+        errors.append(np.linalg.norm(y.cpu().numpy() - want))
+    assert errors[0] <= 1.1 * errors[1]
+
+
 @pytest.mark.parametrize("fmt", FORMATS)
 def test_wide_expert_rows_keep_fp32_activations(device, fmt):
     """Per-route projections wider than the 16-bit kernel takes run on the exact fp32 kernel (2-norm error 4e-7; 16 bits per
@@ -150,3 +190,35 @@ def test_wide_expert_rows_keep_fp32_activations(device, fmt):
     device.synchronize()
     want = np.stack([dense[e] @ x[i].astype(np.float64) for i, e in enumerate(ids)])
     assert np.linalg.norm(y.cpu().numpy() - want) <= 4e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 16])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_infinite_and_nan_activations(device, fmt, m, grouped):
+    """As fp32 products have it: an infinity alone in a row gives infinities with the signs of its weights, infinities of
+    both signs give NaN where their products disagree, a NaN gives NaN, and other rows do not notice."""
+    s = S()
+    rows, cols, inf = 40, 1024, np.float32(np.inf)
+    packed = ref.random_matrix(fmt, rows, cols, seed=8)
+    dense = ref.dequant(fmt, packed).reshape(rows, cols)
+    w = s.Matrix.from_packed(device, rows, cols, 1, fmt, packed)
+    plain = np.random.default_rng(m).standard_normal((m, cols)).astype(np.float32)
+    for row, places in [(0, {5: inf}), (m - 1, {300: -inf}), (0, {5: inf, 6: inf}), (m // 2, {40: inf, 41: -inf, 77: inf}), (0, {5: inf, 900: -inf}),
+                        (m - 1, {1: np.float32(np.nan), 2: inf}), (0, {c: inf for c in range(512, 768)})]:
+        x = plain.copy()
+        for c, v in places.items():
+            x[row, c] = v
+        y = torch.zeros(m, rows, device="cuda")
+        if grouped:
+            s.project_mm_id(device, w, dev_f32(x), dev_u32(np.array([0, m])), m, y)
+        else:
+            s.project(device, w, dev_f32(x), m, y)
+        device.synchronize()
+        with np.errstate(invalid="ignore"):
+            want = np.stack([(dense * r).sum(axis=1, dtype=np.float64) for r in x])
+        got = y.cpu().numpy()
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        assert np.array_equal(np.isinf(got), np.isinf(want)) and np.array_equal(np.sign(got[np.isinf(got)]), np.sign(want[np.isinf(want)]))
+        ok = np.isfinite(want)
+        assert np.allclose(got[ok], want[ok], rtol=0, atol=1e-5 * np.abs(dense).sum(axis=1).max())
