@@ -1144,6 +1144,9 @@ static int moe_experts_f32(fq_device *dev, const fq_moe_ffn_desc *f, const float
     dn.offsets = offsets;
     dn.groups = groups;
     const size_t share = routes * groups / f->experts; // the rows these groups are expected to hold
+    dn.probe = true; // before gate and up are enqueued
+    if (int rc = launch_grouped_f32(dev, &dn, 1, (uint32_t)routes, share, nullptr, 1)) return rc;
+    dn.probe = false;
     if (int rc = launch_grouped_f32(dev, gu, 2, (uint32_t)routes, share, s.sorted, f->used)) return rc;
     return launch_grouped_f32(dev, &dn, 1, (uint32_t)routes, share, nullptr, 1);
 }

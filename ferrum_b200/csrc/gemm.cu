@@ -1406,6 +1406,7 @@ int fq_launch_gemm_f16_grouped(fq_device *dev, const ProjectArgs *a, uint32_t co
     chunk = std::min<uint32_t>(chunk, (G_MAX_TILES - f.groups) * G_TOK); // the kernel's table of activation tiles holds G_MAX_TILES
     if (chunk < total_rows) chunk &= ~(G_TOK - 1);
     if (chunk < 16) return FQ_ERR_UNSUPPORTED;
+    if (f.probe) return FQ_OK;
     __half *xh = (__half *)dev->xprep;
     float *inv_scale = (float *)((uint8_t *)dev->xprep + (size_t)2 * chunk * f.cols * sizeof(__half));
     GJob J{};

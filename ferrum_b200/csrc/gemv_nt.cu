@@ -1009,14 +1009,18 @@ template <int FMT, int NT, bool GROUPED> cudaError_t nt_launch(fq_device *dev, c
     return launch_pdl(kernel, dim3(grid), dim3(S.warps * 32), S.smem, dev->stream, J, push);
 }
 
+bool nt_wide(int format) { return format == FQ_IQ4_XS || format == FQ_IQ4_NL; }
+bool prep_fits(const fq_device *dev, int format, uint32_t cols, uint32_t xrows) {
+    return (size_t)xrows * prep_nt_layout(cols, nt_wide(format)).token_bytes <= dev->xprep_bytes / 2;
+}
 // Prepares `xrows` activation rows into the handle's scratch (its two halves alternate, so a preparation that
 // starts early never writes what the projection before may still be reading) and returns where, or null when
 // they do not fit.
 uint8_t *launch_prep(fq_device *dev, int format, const ProjectArgs &f, uint32_t xrows, const uint32_t *src, uint32_t src_div, const uint32_t *range,
                      uint32_t range_stride, cudaError_t &e) {
-    const bool iq4 = format == FQ_IQ4_XS || format == FQ_IQ4_NL;
+    const bool iq4 = nt_wide(format);
     const PrepNT L = prep_nt_layout(f.cols, iq4);
-    if ((size_t)xrows * L.token_bytes > dev->xprep_bytes / 2) return nullptr;
+    if (!prep_fits(dev, format, f.cols, xrows)) return nullptr;
     dev->xprep_turn ^= 1u;
     uint8_t *prep = (uint8_t *)dev->xprep + (dev->xprep_turn ? dev->xprep_bytes / 2 : 0);
     const dim3 grid(xrows, (L.nblk + PREP_WARPS - 1) / PREP_WARPS);
@@ -1113,16 +1117,18 @@ template <int FMT, int GNT> int launch_grouped(fq_device *dev, NtJob &J, const P
         return FQ_ERR_UNSUPPORTED;
     }
     J.nb_max = S.nb_max;
+    if (src && src_div == 0) return FQ_ERR_UNSUPPORTED;
+    const uint32_t xrows = src ? (J.total_rows + src_div - 1) / src_div : J.total_rows;
+    if (f.probe) return prep_fits(dev, FMT, f.cols, xrows) ? FQ_OK : FQ_ERR_UNSUPPORTED;
     cudaError_t e = cudaSuccess;
     // With a gather (`src`) every row of x is prepared once and the blocks pick rows by index; else the rows of
     // the experts in `offsets` (a rank's share when the matrices hold only some experts).
     if (src) {
-        if (src_div == 0) return FQ_ERR_UNSUPPORTED;
         J.src = src;
         J.src_div = src_div;
-        J.prep = launch_prep(dev, FMT, f, (J.total_rows + src_div - 1) / src_div, nullptr, 1, nullptr, 0, e);
+        J.prep = launch_prep(dev, FMT, f, xrows, nullptr, 1, nullptr, 0, e);
     } else {
-        J.prep = launch_prep(dev, FMT, f, J.total_rows, nullptr, 1, f.offsets, f.groups, e);
+        J.prep = launch_prep(dev, FMT, f, xrows, nullptr, 1, f.offsets, f.groups, e);
     }
     if (!J.prep) return FQ_ERR_UNSUPPORTED;
     if (int rc = fq_check_cuda(dev, e, "activation preparation launch")) return rc;

@@ -146,6 +146,7 @@ struct ProjectArgs {
     const uint32_t *slots = nullptr;
     uint32_t groups = 0, max_rows = 0;
     uint32_t experts = 1;              // expert slices stored in w
+    bool probe = false;                // grouped launchers: answer whether the shape has a kernel (FQ_OK), enqueue nothing
     const CombineTail *combine = nullptr; // project_id of one target, one activation row per route (x_div = 1)
 };
 int fq_launch_project_exact(fq_device *dev, const ProjectArgs &a);

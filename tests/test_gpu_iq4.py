@@ -222,3 +222,22 @@ def test_infinite_and_nan_activations(device, fmt, m, grouped):
         assert np.array_equal(np.isinf(got), np.isinf(want)) and np.array_equal(np.sign(got[np.isinf(got)]), np.sign(want[np.isinf(want)]))
         ok = np.isfinite(want)
         assert np.allclose(got[ok], want[ok], rtol=0, atol=1e-5 * np.abs(dense).sum(axis=1).max())
+
+
+def test_block_whose_down_projection_has_no_grouped_kernel(device):
+    """Gate and up would fit the grouped integer kernel, the wider down projection does not: the block takes the other path
+    from the start, with as many launches as a block none of whose projections fits."""
+    s = S()
+    fmt, experts, used, ffn, m = ref.IQ4_XS, 8, 4, 2816, 21
+    counts = []
+    for hidden in (512, 2816):
+        M = lambda rows, cols, e, f=fmt: s.Matrix.from_packed(device, rows, cols, e, f, ref.random_matrix(f, rows * e, cols, rows + cols))
+        f = s.MoeFfn(M(experts, hidden, 1, ref.Q8_0), M(ffn, hidden, experts), M(ffn, hidden, experts), M(hidden, ffn, experts),
+                     M(256, hidden, 1, ref.Q4_K), M(256, hidden, 1, ref.Q4_K), M(hidden, 256, 1, ref.Q4_K), None, experts, used, hidden, ffn, 256, False, True)
+        scratch, x, out = torch.zeros(s.moe_ffn_scratch_elems(device, f, m), device="cuda"), torch.randn(m, hidden, device="cuda"), torch.zeros(m, hidden, device="cuda")
+        before = device.counters().dispatches
+        s.moe_ffn(device, f, x, m, scratch, out)
+        device.synchronize()
+        counts.append(device.counters().dispatches - before)
+        assert bool(torch.isfinite(out).all())
+    assert counts[0] == counts[1]
