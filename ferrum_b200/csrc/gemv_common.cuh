@@ -218,15 +218,24 @@ __device__ __forceinline__ float norm_finish(const float *part, uint32_t n, floa
     for (uint32_t w = 0; w < NORM_WARPS; w++) ss += part[w];
     return 1.0f / sqrtf(ss / (float)n + eps);
 }
-// By a block of at most sixteen warps (a power of two); `part` holds NORM_WARPS floats of shared memory.  Synchronises.
-__device__ __forceinline__ float block_inv_rms(const float *__restrict__ row, uint32_t n, float eps, float *part) {
-    const uint32_t lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (uint32_t w = threadIdx.x >> 5; w < NORM_WARPS; w += warps) {
-        float ss = 0.f;
+// By a block of W warps; `part` holds NORM_WARPS floats of shared memory.  A warp's virtual warps run side by side, so their
+// loads are in flight together.  Synchronises.
+template <uint32_t W> __device__ __forceinline__ float block_inv_rms(const float *__restrict__ row, uint32_t n, float eps, float *part) {
+    constexpr uint32_t PER = NORM_WARPS / W;
+    static_assert(PER * W == NORM_WARPS, "virtual warps are dealt out evenly");
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float ss[PER];
+#pragma unroll
+    for (uint32_t k = 0; k < PER; k++) ss[k] = 0.f;
 #pragma unroll 4
-        for (uint32_t i = 32 * w + lane; i < n / 4; i += 32 * NORM_WARPS) ss = norm_square(ss, reinterpret_cast<const float4 *>(row)[i]);
-        ss = norm_butterfly(ss);
-        if (lane == 0) part[w] = ss;
+    for (uint32_t i = 32 * warp + lane; i < n / 4; i += 32 * NORM_WARPS)
+#pragma unroll
+        for (uint32_t k = 0; k < PER; k++)
+            if (i + 32 * W * k < n / 4) ss[k] = norm_square(ss[k], reinterpret_cast<const float4 *>(row)[i + 32 * W * k]);
+#pragma unroll
+    for (uint32_t k = 0; k < PER; k++) {
+        ss[k] = norm_butterfly(ss[k]);
+        if (lane == 0) part[warp + W * k] = ss[k];
     }
     __syncthreads();
     return norm_finish(part, n, eps);

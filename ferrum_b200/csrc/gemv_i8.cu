@@ -353,7 +353,7 @@ k_gemv_i8s(const __grid_constant__ SlicedJob J, const __grid_constant__ TpPush P
     const uint32_t seq = P.world > 1 ? tp_seq(P) : 0u;
     {
         __shared__ float norm_part[NORM_WARPS];
-        const float scale = J.norm_w ? block_inv_rms(J.x, J.cols, J.norm_eps, norm_part) : 0.f;
+        const float scale = J.norm_w ? block_inv_rms<16>(J.x, J.cols, J.norm_eps, norm_part) : 0.f;
         // A warp's superblocks two at a time, both fetched before either is worked on (the fetch is an L2 round
         // trip; the widest slice of the 27B layer set gives a warp two superblocks).
         for (uint32_t bb = warp; bb < nb; bb += 2 * W) {

@@ -237,7 +237,7 @@ k_prep_nt(const float *__restrict__ x, const float *__restrict__ x_up, const flo
     if (range && (xr < range[0] || xr >= range[range_stride])) return;
     const size_t srow = src ? src[xr] / src_div : xr;
     __shared__ float norm_part[NORM_WARPS];
-    const float scale = norm_w ? block_inv_rms(x + srow * L.cols, L.cols, eps, norm_part) : 0.f;
+    const float scale = norm_w ? block_inv_rms<PREP_WARPS>(x + srow * L.cols, L.cols, eps, norm_part) : 0.f;
     if (b >= L.nblk) return;
     const size_t at = srow * L.cols + (size_t)b * 256;
     const float4 *sp = reinterpret_cast<const float4 *>(x + at + lane * 8);
@@ -820,10 +820,10 @@ k_nt(const __grid_constant__ NtJob J, const __grid_constant__ TpPush P) {
         __shared__ float norm_part[NORM_WARPS];
         float scale0 = 0.f, scale1 = 0.f; // with a norm there are at most two rows
         if (J.norm_w) {
-            scale0 = block_inv_rms(J.x, J.cols, J.norm_eps, norm_part);
+            scale0 = block_inv_rms<16>(J.x, J.cols, J.norm_eps, norm_part);
             if (m > 1) {
                 __syncthreads();
-                scale1 = block_inv_rms(J.x + J.cols, J.cols, J.norm_eps, norm_part);
+                scale1 = block_inv_rms<16>(J.x + J.cols, J.cols, J.norm_eps, norm_part);
             }
         }
         for (uint32_t i = warp; i < m * nb; i += W) {
