@@ -34,8 +34,9 @@ __device__ __forceinline__ void route_token(float *route_smem, const float *__re
     if (used <= 32) { // what every model has; the scores stay in registers
         uint32_t id = 0;
         float weight = 0.f;
-        const bool good = experts <= 256 ? fqk::route_row<8>(row, experts, used, sigmoid, norm, lane, id, weight)
-                                         : fqk::route_row<32>(row, experts, used, sigmoid, norm, lane, id, weight);
+        const bool good = experts <= 256   ? fqk::route_row<8>(row, experts, used, sigmoid, norm, lane, id, weight)
+                          : experts <= 512 ? fqk::route_row<16>(row, experts, used, sigmoid, norm, lane, id, weight)
+                                           : fqk::route_row<32>(row, experts, used, sigmoid, norm, lane, id, weight);
         // A NaN or an infinity among the logits has no ranking: as below.
         if (!good && lane == 0) *(volatile int *)status = (int)FQ_ERR_WEIGHT;
         if (lane < used) {

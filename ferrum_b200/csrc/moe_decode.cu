@@ -207,8 +207,9 @@ k_moe_decode(const __grid_constant__ MoeDecodeJob J) {
     if (warp == 0) {
         uint32_t id = 0;
         float weight = 0.f;
-        const bool good = J.experts <= 256 ? route_row<8>(J.logits, J.experts, J.used, J.sigmoid, J.norm, lane, id, weight)
-                                           : route_row<32>(J.logits, J.experts, J.used, J.sigmoid, J.norm, lane, id, weight);
+        const bool good = J.experts <= 256   ? route_row<8>(J.logits, J.experts, J.used, J.sigmoid, J.norm, lane, id, weight)
+                          : J.experts <= 512 ? route_row<16>(J.logits, J.experts, J.used, J.sigmoid, J.norm, lane, id, weight)
+                                             : route_row<32>(J.logits, J.experts, J.used, J.sigmoid, J.norm, lane, id, weight);
         if (lane < J.used) { // a row of logits without a ranking: reported, and the token gets weight zero
             ids[lane] = good ? id : lane;
             weights[lane] = good ? weight : 0.f;
