@@ -336,6 +336,17 @@ int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *
         return FQ_ERR_UNSUPPORTED;
     if (H % 256 || F % 256 || SF % 256 || H == 0 || F == 0 || SF == 0 || H > 16384 || f->used == 0 || f->used > MAX_USED || f->experts > 1024 || f->used > f->experts)
         return FQ_ERR_UNSUPPORTED;
+    // In the last phase a warp walks a route's row alone, F / 256 superblocks, and a tile of the shared expert's gate or up
+    // has no more warps than k_gemv_i8s cuts K into slices; the chain deals both out over all SMs.  Wide blocks are its:
+    // one launch against chain, us, Q4_K / Q6_K, 16 experts: H 2048, two routes, F 1024 20.9 / 34.3, 3072 33.6 / 38.7,
+    // 4096 37.7 / 41.4, 8192 66.9 / 52.5; four routes, F 3072 41.2 / 48.7, 4096 51.7 / 51.8; H 4096, one route, F 2048
+    // 35.4 / 40.6, 3072 47.2 / 42.7, eight routes, F 3072 88.2 / 93.1, 4096 113 / 108; shared expert at H 2048, F 1024:
+    // 4096 30.9 / 40.2, 8192 51.0 / 43.5.
+    const uint32_t used = f->used;
+    const uint32_t most_ffn = H <= 2048 ? (used <= 2 ? 4096u : used <= 4 || H > 1024 ? 3072u : 2048u)
+                                        : (used >= 12 ? 4096u : used >= 8 || (used >= 4 && H <= 4096) ? 3072u : 2048u);
+    const uint32_t most_shared = F > 2048 ? 2048u : H <= 2048 ? (used >= 4 ? 6144u : 4096u) : H <= 4096 && F >= 512 ? 4096u : 2048u;
+    if (F > most_ffn || SF > most_shared) return FQ_ERR_UNSUPPORTED;
     if (f->shared_up->rows != SF || f->shared_gate->cols != H || f->shared_up->cols != H || f->shared_down->cols != SF || f->up_exps->cols != H)
         return FQ_ERR_UNSUPPORTED;
     MoeDecodeJob J{};
