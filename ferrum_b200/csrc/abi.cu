@@ -707,15 +707,28 @@ static int check_dtype(fq_device *dev, int dt) {
 
 static bool is_iq4(uint32_t format) { return format == FQ_IQ4_NL || format == FQ_IQ4_XS; }
 
-// Decode / verify widths (F32 in and out): Q8_0 on the integer-dot kernel, Q4_K / Q6_K on the integer tensor
-// path -- one activation row (and per-route expert projections) in gemv_i8.cu, 2..16 rows in gemv_nt.cu.
+// Small IQ4 matrices of more rows than k_nt packs into an MMA tile: its preparation launch and its ring cost more than the
+// whole product on the fp32 kernel (512 x 512, sixteen rows 9.7 -> 6.5 us IQ4_XS, 9.6 -> 8.4 us IQ4_NL; 1024 x 256, eight
+// rows 5.7 -> 4.1 and 5.6 -> 5.2 us; from 2048 x 512 or 1024 columns on k_nt is ahead: sixteen rows 9.9 against 11.8 us).
+static bool iq4_on_fp32(const ProjectArgs &a) {
+    if (a.m < 5 || a.rows > 2048) return false;
+    return a.format == FQ_IQ4_XS ? a.cols <= 512 : a.cols == 256 || (a.cols == 512 && a.rows <= 512 && a.m > 8);
+}
+
+// Decode / verify widths (F32 in and out): Q8_0 on the integer-dot kernel, Q4_K, Q5_K and Q6_K on the integer tensor path
+// -- one activation row (and per-route expert projections) in gemv_i8.cu, 2..16 rows in gemv_nt.cu -- and the IQ4 formats
+// there too, except for routes and one short row (gemv_iq4.cu).
 static int launch_decode(fq_device *dev, const ProjectArgs *a, uint32_t count) {
     if (count == 1 && a[0].format == FQ_Q8_0) {
         int rc = fq_launch_gemv_q8(dev, a[0]);
         if (rc != FQ_ERR_UNSUPPORTED) return rc;
     }
     const bool iq4 = is_iq4(a[0].format);
-    if (count == 1 && a[0].ids && iq4) return fq_launch_gemv_iq4(dev, a[0]);
+    if (count == 1 && iq4 && (a[0].ids || !dev->tp_push)) {
+        int rc = fq_launch_gemv_iq4(dev, a[0]);
+        if (rc != FQ_ERR_UNSUPPORTED || a[0].ids) return rc;
+        if (!a[0].x_up && iq4_on_fp32(a[0])) return FQ_ERR_UNSUPPORTED;
+    }
     if ((a[0].m == 1 && !iq4) || a[0].ids) return fq_launch_gemv_i8_many(dev, a, count);
     return fq_launch_gemv_nt_many(dev, a, count);
 }

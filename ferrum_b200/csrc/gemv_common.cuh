@@ -108,6 +108,26 @@ struct Quant8Wide {
     uint32_t p[4][2]; // values 0-3 and 4-7, one per byte
     float inv;
 };
+// The scale of a group of values from amax, the largest |value| that is no NaN, and whether one is.
+struct WideScale {
+    float s0, s1, inv; // 2^e may be beyond fp32: two factors
+    bool finite, nan;
+    __device__ __forceinline__ WideScale(float amax, bool nan_) : nan(nan_) {
+        finite = amax < INFINITY && !nan;
+        // amax = 1.f * 2^ex: e = 30 - ex, one less where the mantissa is above that of 0x7F7F7F00; a subnormal amax ends at 149.
+        const uint32_t bits = __float_as_uint(amax);
+        int e = 0;
+        if (amax > 0.f && finite) e = min(149, 157 - (int)(bits >> 23) - ((bits & 0x7FFFFFu) > 0x7EFEFEu));
+        inv = e > 126 ? __uint_as_float(1u << (149 - e)) : __uint_as_float((uint32_t)(127 - e) << 23);
+        if (!finite) inv = nan ? __int_as_float(0x7fc00000) : INFINITY;
+        const int e0 = e >> 1;
+        s0 = __uint_as_float((uint32_t)(127 + e0) << 23);
+        s1 = __uint_as_float((uint32_t)(127 + e - e0) << 23);
+    }
+    // A value's digits, the most significant in the top byte (adding 0x80 to every digit makes them unsigned).
+    __device__ __forceinline__ uint32_t digits(float v) const { return ((uint32_t)__float2int_rn(v * s0 * s1) + 0x80808080u) ^ 0x80808080u; }
+    __device__ __forceinline__ uint32_t sign_of_infinity(float v) const { return nan || fabsf(v) < INFINITY ? 0u : v > 0.f ? 0x01000000u : 0xFF000000u; }
+};
 __device__ __forceinline__ Quant8Wide quantize8_wide(const float (&v)[8]) {
     Quant8Wide q;
     float amax = 0.f;
@@ -120,22 +140,14 @@ __device__ __forceinline__ Quant8Wide quantize8_wide(const float (&v)[8]) {
     nan = __any_sync(0xffffffffu, nan);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-    const bool finite = amax < INFINITY && !nan;
-    // amax = 1.f * 2^ex: e = 30 - ex, one less where the mantissa is above that of 0x7F7F7F00; a subnormal amax ends at 149.
-    const uint32_t bits = __float_as_uint(amax);
-    int e = 0;
-    if (amax > 0.f && finite) e = min(149, 157 - (int)(bits >> 23) - ((bits & 0x7FFFFFu) > 0x7EFEFEu));
-    q.inv = e > 126 ? __uint_as_float(1u << (149 - e)) : __uint_as_float((uint32_t)(127 - e) << 23);
-    if (!finite) q.inv = nan ? __int_as_float(0x7fc00000) : INFINITY;
-    // 2^e may be beyond fp32: two factors.
-    const int e0 = e >> 1;
-    const float s0 = __uint_as_float((uint32_t)(127 + e0) << 23), s1 = __uint_as_float((uint32_t)(127 + e - e0) << 23);
-    uint32_t d[8]; // the digits of a value, the most significant in the top byte: adding 0x80 to every digit makes them unsigned
+    const WideScale s(amax, nan);
+    q.inv = s.inv;
+    uint32_t d[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) d[i] = ((uint32_t)__float2int_rn(v[i] * s0 * s1) + 0x80808080u) ^ 0x80808080u;
-    if (!finite)
+    for (int i = 0; i < 8; i++) d[i] = s.digits(v[i]);
+    if (!s.finite)
 #pragma unroll
-        for (int i = 0; i < 8; i++) d[i] = nan || fabsf(v[i]) < INFINITY ? 0u : v[i] > 0.f ? 0x01000000u : 0xFF000000u;
+        for (int i = 0; i < 8; i++) d[i] = s.sign_of_infinity(v[i]);
 #pragma unroll
     for (int h = 0; h < 2; h++) { // bytes of four values -> one word per digit
         const uint32_t *x = d + 4 * h;
