@@ -66,6 +66,7 @@ SIGNATURES = {
     "fq_set_exact": (_I, [_P, _I]),
     "fq_test_fail_after": (_I, [_P, _I]),
     "fq_test_fail_completion": (_I, [_P]),
+    "fq_test_moe_wait": (_I, [_P]),
     "fq_probe_read_stream": (_I, [_P, _P, _Z, _U32]),
     "fq_set_profiling": (_I, [_P, _I]),
     "fq_take_profile": (_I, [_P, C.POINTER(ProfileEntry), _Z, C.POINTER(_Z)]),

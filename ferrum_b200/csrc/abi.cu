@@ -414,6 +414,12 @@ extern "C" int fq_test_fail_after(fq_device *dev, int n) {
     return FQ_OK;
 }
 
+extern "C" int fq_test_moe_wait(fq_device *dev) {
+    if (!dev) return FQ_ERR_PARAM;
+    dev->test_moe_wait = true;
+    return FQ_OK;
+}
+
 extern "C" int fq_test_fail_completion(fq_device *dev) {
     if (!dev) return FQ_ERR_PARAM;
     dev->fail_completion = true;

@@ -34,6 +34,7 @@ struct fq_device {
     bool exact = false;
     int fail_after = -1;          // test hook: enqueues left before an injected failure
     bool fail_completion = false; // test hook: next synchronize reports failure
+    bool test_moe_wait = false;   // test hook: the next one-launch MoE block waits for a block that does not exist
     fq_counters counters{};
     // Output ranges enqueued since the last completion point, and the ranges a failed submission wrote: an input
     // that overlaps one of the latter is refused until a later submission that rewrites it has completed

@@ -34,7 +34,7 @@ using namespace fqk;
 constexpr uint32_t WARPS = 16;
 constexpr uint32_t MAX_USED = 12;    // warps of the last phase: one per route, the rest on the shared expert
 constexpr uint32_t MAX_PARTS = 64;   // partial results of a tile held in shared memory
-constexpr uint64_t WAIT_NS = 2000000000ull;
+constexpr uint64_t WAIT_NS = 2000000000ull, TEST_WAIT_NS = 20000000ull;
 
 struct MoeDecodeJob {
     const float *x, *shared_w; // shared_w null: no gate on the shared expert
@@ -46,13 +46,15 @@ struct MoeDecodeJob {
     uint32_t sg_slices, sd_slices, gu_split, dn_split;
     float *logits, *g, *u, *shared_g, *shared_u; // [experts], [used][ffn] x 2, [shared_ffn] x 2
     uint32_t *barrier;                           // three words, zero between launches
+    uint32_t arrivals;                           // that a barrier waits for: the blocks (a test: one more, so that the wait runs out)
+    uint64_t wait_ns;
     int *status;
 };
 
 __device__ __forceinline__ void prefetch_l2(const uint8_t *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Every block has arrived at `counter` when this returns (or the wait ran out: `gave_up`, for the whole block).
-__device__ __forceinline__ void grid_barrier(uint32_t *counter, int *status, uint32_t &gave_up) {
+__device__ __forceinline__ void grid_barrier(const MoeDecodeJob &J, uint32_t *counter, uint32_t &gave_up) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -62,11 +64,11 @@ __device__ __forceinline__ void grid_barrier(uint32_t *counter, int *status, uin
             for (uint32_t n = 0;; n++) {
                 uint32_t v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-                if (v >= gridDim.x) break;
+                if (v >= J.arrivals) break;
                 if ((n & 255u) == 255u) {
                     if (t0 == 0) t0 = global_ns();
-                    else if (global_ns() - t0 > WAIT_NS) {
-                        *(volatile int *)status = (int)FQ_ERR_TIMEOUT;
+                    else if (global_ns() - t0 > J.wait_ns) {
+                        *(volatile int *)J.status = (int)FQ_ERR_TIMEOUT;
                         gave_up = 1u;
                         break;
                     }
@@ -201,7 +203,7 @@ k_moe_decode(const __grid_constant__ MoeDecodeJob J) {
         }
         __syncthreads();
     }
-    grid_barrier(J.barrier, J.status, gave_up);
+    grid_barrier(J, J.barrier, gave_up);
 
     // ---- phase 1
     if (warp == 0) {
@@ -259,7 +261,7 @@ k_moe_decode(const __grid_constant__ MoeDecodeJob J) {
             __syncthreads();
         }
     }
-    grid_barrier(J.barrier + 1, J.status, gave_up);
+    grid_barrier(J, J.barrier + 1, gave_up);
 
     // ---- phase 2
     for (uint32_t i = warp; i < J.used * fblk; i += WARPS) {
@@ -382,6 +384,8 @@ int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *
     J.shared_g = shared_g;
     J.shared_u = shared_u;
     J.barrier = dev->combine_counters + FQ_COMBINE_COUNTERS;
+    J.arrivals = (uint32_t)dev->sm_count + (dev->test_moe_wait ? 1 : 0);
+    J.wait_ns = dev->test_moe_wait ? TEST_WAIT_NS : WAIT_NS;
     J.status = dev->status_dev;
     const size_t smem = moe_decode_smem(H, F, SF, f->used).total;
     if (smem > 200 * 1024) return FQ_ERR_UNSUPPORTED;
@@ -399,6 +403,7 @@ int fq_launch_moe_decode(fq_device *dev, const fq_moe_ffn_desc *f, const float *
     if (f->shared_gate_inp)
         if (int rc = fq_check_binding(dev, f->shared_gate_inp, (size_t)H * 4, "shared gate weight")) return rc;
     if (int rc = fq_check_no_alias(dev, scratch, scratch_elems * 4, x, (size_t)H * 4, "scratch")) return rc;
+    dev->test_moe_wait = false;
     if (int rc = fq_check_cuda(dev, kernel(dev, J, smem), "moe decode launch")) return rc;
     fq_note_write(dev, out, (size_t)H * 4);
     return fq_end_enqueue(dev, "moe_decode", 1);

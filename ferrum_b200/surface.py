@@ -129,6 +129,9 @@ class Device:
     def fail_completion(self) -> None:
         self.check(self._L.fq_test_fail_completion(self.handle))
 
+    def moe_wait_runs_out(self) -> None:
+        self.check(self._L.fq_test_moe_wait(self.handle))
+
     def set_profiling(self, enabled: bool) -> None:
         """`MetalDevice::set_profiling` (src/metal/mod.rs:636-639): per-operation table on / off, cleared either way."""
         self.check(self._L.fq_set_profiling(self.handle, 1 if enabled else 0))

@@ -88,9 +88,12 @@ int fq_set_exact(fq_device *dev, int on);
 /* Test-only host-side fault injection, the counterpart of `fail_after` / `fail_completion`
  * (src/metal/mod.rs:368-371, 617-620, 846-853): the n-th enqueue from now fails with
  * FQ_ERR_SYNC before anything is launched (n < 0 disarms); `fq_test_fail_completion` makes the
- * next `fq_synchronize` report a failure.  No GPU fault is produced. */
+ * next `fq_synchronize` report a failure; `fq_test_moe_wait` makes the grid barriers of the next one-token MoE block
+ * wait for one block too many, for 20 ms, after which the kernel ends and reports FQ_ERR_TIMEOUT.  No GPU fault is
+ * produced. */
 int fq_test_fail_after(fq_device *dev, int n);
 int fq_test_fail_completion(fq_device *dev);
+int fq_test_moe_wait(fq_device *dev);
 
 /* Opt-in per-operation measurements, the counterpart of `set_profiling` / `take_profile` / `ProfileEntry`
  * (src/metal/mod.rs:636-676, 231-242).  While profiling is on every enqueue is bracketed by a pair of CUDA

@@ -95,3 +95,23 @@ def test_operands_inside_the_scratch(device, inside):
     s.moe_ffn(device, f, x, 1, scratch, out)
     device.synchronize()
     assert torch.equal(out, want) and bool(want.abs().max() > 0)
+
+
+def test_wait_for_the_other_blocks_is_bounded(device):
+    """A barrier that nobody completes gives up after its time, the kernel ends and reports it, and the next block runs."""
+    s = S()
+    f = block(s, device, ref.Q4_K, ref.Q6_K, 16, 4, 512, 256, 256, False, False)
+    x = torch.from_numpy((np.random.default_rng(2).standard_normal(512) * 0.12).astype(np.float32)).cuda()
+    scratch = torch.zeros(s.moe_ffn_scratch_elems(device, f, 1), device="cuda")
+    want, out = torch.zeros(512, device="cuda"), torch.zeros(512, device="cuda")
+    s.moe_ffn(device, f, x, 1, scratch, want)
+    device.synchronize()
+    device.moe_wait_runs_out()
+    s.moe_ffn(device, f, x, 1, scratch, out)
+    with pytest.raises(s.TimeoutError_):
+        device.synchronize()
+    device.recover()
+    out.zero_()
+    s.moe_ffn(device, f, x, 1, scratch, out)
+    device.synchronize()
+    assert torch.equal(out, want)
