@@ -224,10 +224,11 @@ __device__ __forceinline__ float norm_butterfly(float ss) {
     for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
     return ss;
 }
-__device__ __forceinline__ float norm_finish(const float *part, uint32_t n, float eps) {
+// `parts`: the virtual warps the row reaches, where that is known (the others would add zero).
+template <uint32_t parts = NORM_WARPS> __device__ __forceinline__ float norm_finish(const float *part, uint32_t n, float eps) {
     float ss = 0.f;
 #pragma unroll
-    for (uint32_t w = 0; w < NORM_WARPS; w++) ss += part[w];
+    for (uint32_t w = 0; w < parts; w++) ss += part[w];
     return 1.0f / sqrtf(ss / (float)n + eps);
 }
 // By a block of W warps; `part` holds NORM_WARPS floats of shared memory.  A warp's virtual warps run side by side, so their

@@ -6,6 +6,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <utility>
 
 #include "gemv_common.cuh"
@@ -14,65 +15,128 @@
 namespace {
 using namespace fqk;
 
-// One block per row.  Its values stay in registers between the sum and the scaling (rows up to 16384 values; longer
-// ones are read again), every load of a thread is in flight at once, and the launch overlaps the end of the kernel
-// before it.  A decode step's row is latency-bound: 17-22 us with one warp walking the row, about 3 us so.
-constexpr int NORM_CACHED = 8; // float4s a thread keeps
-__global__ void __launch_bounds__(NORM_WARPS * 32)
-k_rmsnorm(const float *x, const float *r, const float *__restrict__ w, uint32_t n, float eps, float *h, float *y) {
+// WPR warps per row.  A row's values stay in registers between the sum and the scaling (CACHED float4s a thread; longer
+// rows are read again), every load of a thread is in flight at once, and the launch overlaps the end of the kernel before
+// it.  The sum is that of sixteen virtual warps (gemv_common.cuh) whatever WPR, so the bits do not depend on it.
+template <int WPR, int CACHED> constexpr int NORM_BLOCK = WPR == 16 ? 16 : WPR == 8 || CACHED <= 2 ? 8 : 4; // warps
+template <int WPR, int CACHED>
+__global__ void __launch_bounds__(NORM_BLOCK<WPR, CACHED> * 32)
+k_rmsnorm(const float *x, const float *r, const float *w, uint32_t n, float eps, uint32_t rows, float *h, float *y) {
     pdl_trigger();
-    // x and r are the outputs of kernels that may still run when this grid starts: coherent loads after the wait.  h may be
+    // x, r and w may be the outputs of kernels that still run when this grid starts: coherent loads after the wait (through
+    // L1 for the weights, which every row reads).  h may be
     // x, and y may be x or r: every value of a row is read before the first of its y is written, and a value's h by the
     // thread that read it.
     pdl_wait();
-    __shared__ float part[NORM_WARPS];
-    constexpr uint32_t T = NORM_WARPS * 32;
-    const uint32_t tid = threadIdx.x, n4 = n / 4;
-    const size_t base = (size_t)blockIdx.x * n4;
+    // Warps of a block; virtual warps of a warp, as far as the row reaches (a row that is all cached may be shorter).
+    constexpr uint32_t W = NORM_BLOCK<WPR, CACHED>, PER = CACHED < NORM_WARPS / WPR ? CACHED : NORM_WARPS / WPR;
+    constexpr bool TAIL = CACHED >= NORM_WARPS / WPR;
+    __shared__ float part[W / WPR][NORM_WARPS];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n4 = n / 4, slot = warp / WPR;
+    const uint32_t row = blockIdx.x * (W / WPR) + slot;
+    const bool live = row < rows;
+    const size_t base = (size_t)(live ? row : 0) * n4;
+    const uint32_t first = 32 * (warp % WPR) + lane, end = live ? n4 : 0;
     const float4 *xr = reinterpret_cast<const float4 *>(x) + base, *rr = r ? reinterpret_cast<const float4 *>(r) + base : nullptr;
     float4 *hr = r ? reinterpret_cast<float4 *>(h) + base : nullptr, *yr = reinterpret_cast<float4 *>(y) + base;
     const float4 *g = reinterpret_cast<const float4 *>(w);
     auto sum = [](const float4 &a, const float4 &b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); };
-    float4 v[NORM_CACHED];
+    float4 v[CACHED]; // value j is the thread's j-th float4 of the row: virtual warp j % PER, its step j / PER
 #pragma unroll
-    for (int j = 0; j < NORM_CACHED; j++) {
-        const uint32_t i = tid + T * j;
-        if (i < n4) v[j] = __ldcg(xr + i);
+    for (int j = 0; j < CACHED; j++) {
+        const uint32_t i = first + 32 * WPR * j;
+        if (i < end) v[j] = __ldcg(xr + i);
     }
     if (r) { // h = x + r first; the norm is taken of h
 #pragma unroll
-        for (int j = 0; j < NORM_CACHED; j++) {
-            const uint32_t i = tid + T * j;
-            if (i < n4) v[j] = sum(v[j], __ldcg(rr + i));
+        for (int j = 0; j < CACHED; j++) {
+            const uint32_t i = first + 32 * WPR * j;
+            if (i < end) v[j] = sum(v[j], __ldcg(rr + i));
         }
     }
-    float ss = 0.f;
+    float4 gv[CACHED]; // the weights are on their way while the sum is taken
 #pragma unroll
-    for (int j = 0; j < NORM_CACHED; j++) {
-        const uint32_t i = tid + T * j;
-        if (i < n4) {
+    for (int j = 0; j < CACHED; j++) {
+        const uint32_t i = first + 32 * WPR * j;
+        if (i < end) gv[j] = g[i];
+    }
+    float ss[PER];
+#pragma unroll
+    for (uint32_t k = 0; k < PER; k++) ss[k] = 0.f;
+#pragma unroll
+    for (int j = 0; j < CACHED; j++) {
+        const uint32_t i = first + 32 * WPR * j;
+        if (i < end) {
             if (r) hr[i] = v[j];
-            ss = norm_square(ss, v[j]);
+            ss[j % PER] = norm_square(ss[j % PER], v[j]);
         }
     }
-    for (uint32_t i = tid + T * NORM_CACHED; i < n4; i += T) {
-        float4 a = __ldcg(xr + i);
-        if (r) hr[i] = a = sum(a, __ldcg(rr + i));
-        ss = norm_square(ss, a);
+    static_assert(!TAIL || CACHED % PER == 0, "the tail starts with virtual warp 0 of the warp");
+    if constexpr (TAIL)
+        for (uint32_t i0 = first + 32 * WPR * CACHED; i0 < end; i0 += 32 * NORM_WARPS)
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) {
+                const uint32_t i = i0 + 32 * WPR * k;
+                if (i < end) {
+                    float4 a = __ldcg(xr + i);
+                    if (r) hr[i] = a = sum(a, __ldcg(rr + i));
+                    ss[k] = norm_square(ss[k], a);
+                }
+            }
+    float scale;
+    if constexpr (WPR == 1) {
+        // The sums of all virtual warps at once: the same butterfly steps, but at each a lane keeps only the half of the
+        // sums that its bit picks, so that sum k ends in the lanes from k * 32 / PER on.
+        uint32_t off = 16;
+#pragma unroll
+        for (uint32_t half = PER / 2; half > 0; half /= 2, off /= 2)
+#pragma unroll
+            for (uint32_t k = 0; k < half; k++) {
+                const float give = (lane & off) ? ss[k] : ss[k + half], keep = (lane & off) ? ss[k + half] : ss[k];
+                ss[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+            }
+#pragma unroll
+        for (; off > 0; off /= 2) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], off);
+        float sums[PER];
+#pragma unroll
+        for (uint32_t k = 0; k < PER; k++) sums[k] = __shfl_sync(0xffffffffu, ss[0], k * (32 / PER));
+        scale = norm_finish<PER>(sums, n, eps);
+    } else {
+#pragma unroll
+        for (uint32_t k = 0; k < PER; k++) ss[k] = norm_butterfly(ss[k]);
+        if (lane == 0)
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) part[slot][warp % WPR + WPR * k] = ss[k];
+        __syncthreads();
+        scale = norm_finish(part[slot], n, eps);
     }
-    ss = norm_butterfly(ss);
-    if ((tid & 31) == 0) part[tid >> 5] = ss;
-    __syncthreads();
-    const float scale = norm_finish(part, n, eps);
     auto scaled = [scale](const float4 &a, const float4 &b) {
         return make_float4(a.x * scale * b.x, a.y * scale * b.y, a.z * scale * b.z, a.w * scale * b.w);
     };
 #pragma unroll
-    for (int j = 0; j < NORM_CACHED; j++) {
-        const uint32_t i = tid + T * j;
-        if (i < n4) yr[i] = scaled(v[j], g[i]);
+    for (int j = 0; j < CACHED; j++) {
+        const uint32_t i = first + 32 * WPR * j;
+        if (i < end) yr[i] = scaled(v[j], gv[j]);
     }
-    for (uint32_t i = tid + T * NORM_CACHED; i < n4; i += T) yr[i] = scaled(__ldcg((r ? hr : xr) + i), g[i]);
+    if constexpr (TAIL)
+        for (uint32_t i = first + 32 * WPR * CACHED; i < end; i += 32 * WPR) yr[i] = scaled(__ldcg((r ? hr : xr) + i), g[i]);
+}
+
+cudaError_t launch_norm(fq_device *dev, const float *x, const float *r, const float *w, uint32_t n, float eps, uint32_t rows, float *h, float *y) {
+    auto go = [&](auto wpr, auto cached) {
+        constexpr int WPR = decltype(wpr)::value, C = decltype(cached)::value, W = NORM_BLOCK<WPR, C>;
+        return launch_pdl(k_rmsnorm<WPR, C>, dim3((rows + W / WPR - 1) / (W / WPR)), dim3(W * 32), 0, dev->stream, x, r, w, n, eps, rows, h, y);
+    };
+    using std::integral_constant;
+    constexpr integral_constant<int, 1> one;
+    constexpr integral_constant<int, 2> two;
+    constexpr integral_constant<int, 4> four;
+    constexpr integral_constant<int, 8> eight;
+    if (rows <= 2 * (uint32_t)dev->sm_count || n > 8192) return go(integral_constant<int, 16>{}, eight);
+    if (n > 4096) return go(eight, eight);
+    if (n > 2048) return go(four, eight);
+    if (n > 1024) return go(two, eight);
+    return n > 512 ? go(one, eight) : n > 256 ? go(one, four) : n > 128 ? go(one, two) : go(one, one);
 }
 
 __device__ __forceinline__ void better(float &bv, uint32_t &bi, float ov, uint32_t oi) {
@@ -210,9 +274,7 @@ int check_norm(fq_device *dev, const float *x, const float *w, uint32_t n, uint3
 extern "C" int fq_rmsnorm(fq_device *dev, const float *x, const float *w, uint32_t n, float eps, uint32_t rows, float *y) {
     if (int rc = fq_begin_enqueue(dev)) return rc;
     if (int rc = check_norm(dev, x, w, n, rows, y)) return rc;
-    if (int rc = fq_check_cuda(dev, launch_pdl(k_rmsnorm, dim3(rows), dim3(NORM_WARPS * 32), 0, dev->stream, x, (const float *)nullptr, w, n, eps, (float *)nullptr, y),
-                               "rmsnorm launch"))
-        return rc;
+    if (int rc = fq_check_cuda(dev, launch_norm(dev, x, nullptr, w, n, eps, rows, nullptr, y), "rmsnorm launch")) return rc;
     return fq_end_enqueue(dev, "rmsnorm", 1);
 }
 
@@ -223,7 +285,7 @@ extern "C" int fq_add_rmsnorm(fq_device *dev, const float *x, const float *r, co
     if (int rc = fq_check_binding(dev, r, (size_t)rows * n * 4, "r")) return rc;
     if (int rc = fq_check_binding(dev, h, (size_t)rows * n * 4, "h")) return rc;
     if (int rc = fq_check_no_alias(dev, y, (size_t)rows * n * 4, h, (size_t)rows * n * 4, "y")) return rc;
-    if (int rc = fq_check_cuda(dev, launch_pdl(k_rmsnorm, dim3(rows), dim3(NORM_WARPS * 32), 0, dev->stream, x, r, w, n, eps, h, y), "add_rmsnorm launch")) return rc;
+    if (int rc = fq_check_cuda(dev, launch_norm(dev, x, r, w, n, eps, rows, h, y), "add_rmsnorm launch")) return rc;
     return fq_end_enqueue(dev, "add_rmsnorm", 1);
 }
 
