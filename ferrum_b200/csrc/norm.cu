@@ -146,6 +146,33 @@ __device__ __forceinline__ void better(float &bv, uint32_t &bi, float ov, uint32
     }
 }
 
+// Float groups first, first + step, .. below `groups` of a row: the first maximum of a thread's share so far.
+template <int VEC>
+__device__ __forceinline__ void argmax_scan(const float *x, uint32_t first, uint32_t groups, uint32_t step, float &bv, uint32_t &bi) {
+    auto take = [&](float v, uint32_t i) {
+        if (v > bv) {
+            bv = v;
+            bi = i;
+        }
+    };
+#pragma unroll 4
+    for (uint32_t i = first; i < groups; i += step) {
+        if constexpr (VEC == 4) {
+            const float4 v = reinterpret_cast<const float4 *>(x)[i];
+            take(v.x, 4 * i);
+            take(v.y, 4 * i + 1);
+            take(v.z, 4 * i + 2);
+            take(v.w, 4 * i + 3);
+        } else {
+            take(x[i], i);
+        }
+    }
+}
+template <int LANES> __device__ __forceinline__ void argmax_reduce(float &bv, uint32_t &bi) {
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) better(bv, bi, __shfl_down_sync(0xffffffffu, bv, off), __shfl_down_sync(0xffffffffu, bi, off));
+}
+
 // The index of the first maximum of a row, by a cluster of eight blocks: each takes a contiguous part of the row and
 // block 0 collects the parts' winners through distributed shared memory (a 151,936-value row of logits: 7.8 us with
 // one block, whose single SM is what bounds it).  VEC: values per load (4 where rows start on 16-byte boundaries).
@@ -170,28 +197,8 @@ k_argmax(const float *x, uint32_t n, uint32_t *out) {
     const uint32_t end = min(groups, (rank + 1) * per);
     float bv = -INFINITY;
     uint32_t bi = 0;
-    auto take = [&](float v, uint32_t i) {
-        if (v > bv) {
-            bv = v;
-            bi = i;
-        }
-    };
-#pragma unroll 4
-    for (uint32_t i = rank * per + tid; i < end; i += 512) {
-        if constexpr (VEC == 4) {
-            const float4 v = __ldcg(reinterpret_cast<const float4 *>(x) + i);
-            take(v.x, 4 * i);
-            take(v.y, 4 * i + 1);
-            take(v.z, 4 * i + 2);
-            take(v.w, 4 * i + 3);
-        } else {
-            take(__ldcg(x + i), i);
-        }
-    }
-    auto reduce = [&](int lanes) {
-        for (int off = lanes / 2; off > 0; off >>= 1) better(bv, bi, __shfl_down_sync(0xffffffffu, bv, off), __shfl_down_sync(0xffffffffu, bi, off));
-    };
-    reduce(32);
+    argmax_scan<VEC>(x, rank * per + tid, end, 512, bv, bi);
+    argmax_reduce<32>(bv, bi);
     if ((tid & 31) == 0) {
         best_v[tid >> 5] = bv;
         best_i[tid >> 5] = bi;
@@ -201,7 +208,7 @@ k_argmax(const float *x, uint32_t n, uint32_t *out) {
     if (tid < 32) {
         bv = best_v[tid & 15];
         bi = best_i[tid & 15];
-        reduce(16);
+        argmax_reduce<16>(bv, bi);
         if (tid == 0) {
             cluster.map_shared_rank(part_v, 0)[rank] = bv;
             cluster.map_shared_rank(part_i, 0)[rank] = bi;
@@ -211,9 +218,39 @@ k_argmax(const float *x, uint32_t n, uint32_t *out) {
     if (rank == 0 && tid < 32) {
         bv = part_v[tid & 7];
         bi = part_i[tid & 7];
-        reduce(8);
+        argmax_reduce<8>(bv, bi);
         if (tid == 0) out[blockIdx.y] = bi;
     }
+}
+
+// The same by WPR warps per row, without a cluster.
+template <int VEC, int WPR>
+__global__ void __launch_bounds__(WPR == 32 ? 1024 : 256)
+k_argmax_rows(const float *x, uint32_t n, uint32_t rows, uint32_t *out) {
+    pdl_trigger();
+    pdl_wait(); // as above
+    constexpr uint32_t W = WPR == 32 ? 32 : 8;
+    __shared__ float best_v[W];
+    __shared__ uint32_t best_i[W];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.x * (W / WPR) + warp / WPR;
+    if (row >= rows) return; // whole warps, and with several per row whole blocks
+    x += (size_t)row * n;
+    float bv = -INFINITY;
+    uint32_t bi = 0;
+    argmax_scan<VEC>(x, 32 * (warp % WPR) + lane, (n + VEC - 1) / VEC, 32 * WPR, bv, bi);
+    argmax_reduce<32>(bv, bi);
+    if constexpr (WPR > 1) {
+        if (lane == 0) {
+            best_v[warp] = bv;
+            best_i[warp] = bi;
+        }
+        __syncthreads();
+        if (warp != 0) return;
+        bv = best_v[lane % WPR];
+        bi = best_i[lane % WPR];
+        argmax_reduce<WPR>(bv, bi);
+    }
+    if (lane == 0) out[row] = bi;
 }
 
 // grid (ceil(n / 1024), rows), 256 threads: per 1024-value block the 32 largest (value, index) pairs in descending
@@ -294,6 +331,19 @@ extern "C" int fq_argmax(fq_device *dev, const float *x, uint32_t n, uint32_t ro
     if (n == 0 || rows == 0) return fq_fail(dev, FQ_ERR_SHAPE, "argmax of %u rows of %u values", rows, n);
     if (int rc = fq_check_binding(dev, x, (size_t)rows * n * 4, "x")) return rc;
     if (int rc = fq_check_binding(dev, out, (size_t)rows * 4, "out")) return rc;
+    const bool cluster = (n >= 16384 && rows <= 16) || (n >= 65536 && rows <= 64);
+    if (!cluster) {
+        const int shape = n <= 128 || (n <= 2048 && rows >= 1024) ? 1 : n < 12288 ? 8 : 32; // warps per row
+        auto go = [&](auto vec) {
+            constexpr int VEC = decltype(vec)::value;
+            return shape == 1   ? launch_pdl(k_argmax_rows<VEC, 1>, dim3((rows + 7) / 8), dim3(256), 0, dev->stream, x, n, rows, out)
+                   : shape == 8 ? launch_pdl(k_argmax_rows<VEC, 8>, dim3(rows), dim3(256), 0, dev->stream, x, n, rows, out)
+                                : launch_pdl(k_argmax_rows<VEC, 32>, dim3(rows), dim3(1024), 0, dev->stream, x, n, rows, out);
+        };
+        const cudaError_t e = n % 4 == 0 ? go(std::integral_constant<int, 4>{}) : go(std::integral_constant<int, 1>{});
+        if (int rc = fq_check_cuda(dev, e, "argmax launch")) return rc;
+        return fq_end_enqueue(dev, "argmax", 1);
+    }
     for (uint32_t r0 = 0; r0 < rows; r0 += 65535) { // rows sit in the grid's y extent
         const dim3 grid(ARGMAX_CLUSTER, std::min(rows - r0, 65535u));
         const float *xr = x + (size_t)r0 * n;
