@@ -109,8 +109,9 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 }
 
 // One lane of a converged warp.  The branches that issue TMA and MMA instructions are taken by it, not by `lane == 0`: the
-// compiler then knows that a single thread runs them and feeds their uniform operands without a loop over lanes (four
-// prompt projections of 2048 rows 1437 -> 1290 us).
+// compiler then knows that a single thread runs them and feeds their uniform operands without a loop over lanes (the
+// seven projections of a 27B-class layer, 2048 rows: 1437 -> 1290 us; in a bare loop of MMAs the branch costs 53 cycles
+// each, elect.sync 40 at N = 32, and nothing from N = 128 on, where the MMA itself takes longer).
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
@@ -736,9 +737,9 @@ int launch_dense(fq_device *dev, const ProjectArgs &a, const void *x, uint32_t m
 //
 //   y[t][n] = (sum_k (hi[t][k] + lo[t][k]) * fp16(W[e][n][k])) / s[t]      hi + lo = s[t] x[t] to 22 bits
 //
-// A tcgen05.mma with M = 128 takes about the same time whatever its N (measured: N = 32, 80 and 128 alike), so the
-// few activation rows go on the M side -- 64 rows, each as two MMA rows (hi, lo) -- and 256 weight rows on the
-// N side: the widest instruction, the most weights per tensor-core cycle.
+// A tcgen05.mma with M = 128, K = 16 takes 40 / 48 / 64 / 128 cycles at N = 32 / 64 / 128 / 256 (measured back to back), so
+// the full rate starts at N = 128: the few activation rows go on the M side -- 64 rows, each as two MMA rows (hi, lo) --
+// and 256 weight rows on the N side.
 //
 // The block is persistent (one per SM) and walks work items (activation tile of <= 64 expert-sorted rows,
 // 256 weight rows of one of up to two matrix sets) in a strided order:

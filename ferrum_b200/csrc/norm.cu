@@ -132,6 +132,9 @@ cudaError_t launch_norm(fq_device *dev, const float *x, const float *r, const fl
     constexpr integral_constant<int, 2> two;
     constexpr integral_constant<int, 4> four;
     constexpr integral_constant<int, 8> eight;
+    // A few rows, a decode step's, are bound by latency: sixteen warps a row (1 x 5120 1.9 us; one warp 11).  With more rows
+    // than two per SM the machine is full anyway and a row takes the warps its values keep busy: us with that many against
+    // sixteen, 16384 x 128 4.7 / 78, 1024 x 2048 3.9 / 6.5, 2048 x 4096 8.9 / 13.0, 1024 x 5120 6.9 / 10.5.
     if (rows <= 2 * (uint32_t)dev->sm_count || n > 8192) return go(integral_constant<int, 16>{}, eight);
     if (n > 4096) return go(eight, eight);
     if (n > 2048) return go(four, eight);
@@ -331,6 +334,8 @@ extern "C" int fq_argmax(fq_device *dev, const float *x, uint32_t n, uint32_t ro
     if (n == 0 || rows == 0) return fq_fail(dev, FQ_ERR_SHAPE, "argmax of %u rows of %u values", rows, n);
     if (int rc = fq_check_binding(dev, x, (size_t)rows * n * 4, "x")) return rc;
     if (int rc = fq_check_binding(dev, out, (size_t)rows * 4, "out")) return rc;
+    // us with a cluster / one / eight / 32 warps: 1 x 151936 2.7 / 70 / 10 / 4.9, 64 x 151936 5.1 / 72 / 11 / 7.2, 32 x 32000
+    // 2.8 / 16 / 3.7 / 2.6, 148 x 8192 6.3 / 5.0 / 1.9 / 2.1, 1024 x 1024 31 / 1.8 / 2.3 / 5.2, 64 x 256 2.5 / 1.4 / 1.4 / 1.6.
     const bool cluster = (n >= 16384 && rows <= 16) || (n >= 65536 && rows <= 64);
     if (!cluster) {
         const int shape = n <= 128 || (n <= 2048 && rows >= 1024) ? 1 : n < 12288 ? 8 : 32; // warps per row
